@@ -435,7 +435,7 @@ def measure_fused(name, args, torch, stream, flush, world=1, rank=0, local=0, he
         torch.distributed.all_reduce(t, op=torch.distributed.ReduceOp.MAX)
     ms_per_step = float(t.item()) / steps
     peak, peak_kind = load_peak()
-    launches = run.launches_per_step
+    launches = run.kernels_per_step
     alg_bytes = total * (b0 + b1) + n * (12 + (0 if masks is None else 1)) + (n + 1) * 8
     kernel_ms = statistics.median(step_ms)
     achieved = alg_bytes / (kernel_ms / 1e3) / 1e9

@@ -78,12 +78,14 @@ struct vox_ctx {
   int batch_grid[4] = {0, 0, 0, 0};   // persistent grid per gen mode (look-back kernel)
   int phased_grid[4] = {0, 0, 0, 0};  // co-resident grid per gen mode (phased kernel)
   int overlap_grid[4] = {0, 0, 0, 0}; // persistent grid per gen mode (overlap kernel)
+  int emit_grid = 0;                  // persistent grid of the list emission
   int host_grid[4] = {0, 0, 0, 0};    // grid of launches that write host memory (staged)
   // phased and overlap schedules: per-chunk occupancy + halo spill and face totals
   uint32_t* d_scratch = nullptr;
   uint32_t* d_counts = nullptr;
-  size_t scratch_cap = 0;  // chunks
+  size_t scratch_bytes = 0, counts_cap = 0;
   TablesDev* d_tables = nullptr;
+  float2* d_grad2 = nullptr;
   TablesDev h_tables{};  // the fused batch kernels take the tables as a kernel parameter
   BatchCtl* d_ctl = nullptr;
   BatchCtl* h_ctl = nullptr;  // pinned
@@ -270,31 +272,47 @@ int apply_tuning(vox_ctx* ctx, int topt, int stage_faces, int ctas_per_sm, int s
   return VOX_OK;
 }
 
-// Scratch of the phased schedule for n chunks (grows; never shrinks).
-int ensure_scratch(vox_ctx* ctx, size_t n) {
-  if (n <= ctx->scratch_cap) return VOX_OK;
+// Whether a launch goes through the face lists (vox_lists.cuh): the overlap schedule with
+// outputs in device memory, unless the voxels are random, whose chunks never fit a list.
+bool use_lists(const vox_ctx* ctx, int gm, bool host_out) {
+  return ctx->schedule == VOX_SCHEDULE_OVERLAP && !host_out && gm != GM_BERNOULLI;
+}
+
+// Scratch of one chunk of a launch.
+size_t slot_bytes(const vox_ctx* ctx, int gm, bool host_out) {
+  return (size_t)(use_lists(ctx, gm, host_out) ? ctx->ks->list_slot_bytes : ctx->ks->spill_bytes);
+}
+
+// Per-chunk scratch and face totals for n chunks (grow; never shrink).
+int ensure_scratch(vox_ctx* ctx, size_t n, size_t slot) {
   const size_t cap = std::max<size_t>(n, 1024);
-  cudaFree(ctx->d_scratch);
-  cudaFree(ctx->d_counts);
-  ctx->d_scratch = nullptr;
-  ctx->d_counts = nullptr;
-  ctx->scratch_cap = 0;
-  VOX_CUDA(ctx, cudaMalloc(&ctx->d_scratch, cap * (size_t)ctx->ks->spill_bytes),
-           "cudaMalloc(scratch)");
-  VOX_CUDA(ctx, cudaMalloc(&ctx->d_counts, cap * sizeof(uint32_t)), "cudaMalloc(counts)");
-  ctx->scratch_cap = cap;
+  if (n * slot > ctx->scratch_bytes) {
+    cudaFree(ctx->d_scratch);
+    ctx->d_scratch = nullptr;
+    ctx->scratch_bytes = 0;
+    VOX_CUDA(ctx, cudaMalloc(&ctx->d_scratch, cap * slot), "cudaMalloc(scratch)");
+    ctx->scratch_bytes = cap * slot;
+  }
+  if (n > ctx->counts_cap) {
+    cudaFree(ctx->d_counts);
+    ctx->d_counts = nullptr;
+    ctx->counts_cap = 0;
+    VOX_CUDA(ctx, cudaMalloc(&ctx->d_counts, cap * sizeof(uint32_t)), "cudaMalloc(counts)");
+    ctx->counts_cap = cap;
+  }
   return VOX_OK;
 }
 
+// Look-back states of a launch of n chunks (see state_words).
 int ensure_state(vox_ctx* ctx, size_t n) {
   if (n <= ctx->state_cap) return VOX_OK;
-  size_t cap = std::max<size_t>(n, 1024);
+  const size_t cap = std::max<size_t>(n, 1024);
+  const size_t bytes = (size_t)state_words(cap) * sizeof(unsigned long long);
   if (ctx->d_state) cudaFree(ctx->d_state);
   ctx->d_state = nullptr;
   ctx->state_cap = 0;
-  VOX_CUDA(ctx, cudaMalloc(&ctx->d_state, cap * sizeof(unsigned long long)), "cudaMalloc(state)");
-  VOX_CUDA(ctx, cudaMemsetAsync(ctx->d_state, 0, cap * sizeof(unsigned long long), ctx->stream),
-           "cudaMemsetAsync(state)");
+  VOX_CUDA(ctx, cudaMalloc(&ctx->d_state, bytes), "cudaMalloc(state)");
+  VOX_CUDA(ctx, cudaMemsetAsync(ctx->d_state, 0, bytes, ctx->stream), "cudaMemsetAsync(state)");
   ctx->state_cap = cap;
   return VOX_OK;
 }
@@ -305,7 +323,8 @@ int ensure_state(vox_ctx* ctx, size_t n) {
 constexpr unsigned long long kStateWipePeriod = 1ull << 22;
 int before_batch_launch(vox_ctx* ctx) {
   if (ctx->launches > 0 && (ctx->launches & (kStateWipePeriod - 1)) == 0 && ctx->d_state) {
-    VOX_CUDA(ctx, cudaMemsetAsync(ctx->d_state, 0, ctx->state_cap * sizeof(unsigned long long),
+    VOX_CUDA(ctx, cudaMemsetAsync(ctx->d_state, 0,
+                                  (size_t)state_words(ctx->state_cap) * sizeof(unsigned long long),
                                   ctx->stream),
              "cudaMemsetAsync(state)");
   }
@@ -317,8 +336,8 @@ MeshArgs base_args(vox_ctx* ctx) {
   MeshArgs a;
   std::memset(&a, 0, sizeof a);
   a.tables = ctx->d_tables;
+  a.grad2 = ctx->d_grad2;
   a.ctl = ctx->d_ctl;
-  a.state = ctx->d_state;
   a.gen = ctx->gen;
   a.full6 = ctx->cfg.cull_mode == VOX_CULL_FULL6 ? 1 : 0;
   a.stage_faces = ctx->stage_faces;
@@ -350,9 +369,52 @@ int check_outputs(vox_ctx* ctx, void* out0, void* out1, uint64_t cap) {
   return VOX_OK;
 }
 
+// Issues a batch through the face lists: one CTA per chunk lists its faces, then the persistent
+// emission grid writes the records, launched as a programmatic dependent of the first (it
+// starts as the last generation CTAs run, and waits for single chunks). A chunk's faces go out
+// in 2^a.split parts, a warp each: enough to give every resident warp one part (two from 32^3 on,
+// whose chunks are less even), but no fewer than one per 8 (up to 16^3) or 16 output lines
+// of a chunk with two faces a column, and no more than one per 2 or 4 lines. Measured, us a batch
+// with 2, 4, 8, 16, 32 parts: 1024 terrain chunks of 16^3 41, 35, 34, 34, 38; 777 cave chunks
+// of 32^3 from occupancy 56, 51, 46, 42, 41; 64 chunks of 32^3, instances 34, 27, 23, 22, 21.
+int issue_lists(vox_ctx* ctx, MeshArgs& a, int gm, cudaStream_t stream) {
+  const KernelSet& ks = *ctx->ks;
+  const int warps = ks.emit_threads / 32, N = ks.n_size;
+  const bool small = N <= 16;
+  const long long area = (long long)N * N / 8;  // output lines of two faces a column
+  const long long least = std::max<long long>(1, area / (small ? 8 : 16));
+  const long long most = std::max(least, area / (small ? 2 : 4));
+  const long long want = ((small ? 1ll : 2ll) * ctx->emit_grid * warps + a.n - 1) / a.n;
+  const long long parts = std::min(std::max(want, least), most);
+  a.split = 0;
+  while ((1ll << a.split) < parts) ++a.split;
+  const long long scans = ((long long)a.n + (long long)kStateGroup - 1) / (long long)kStateGroup;
+  const long long ctas = std::max(scans, (((long long)a.n << a.split) + warps - 1) / warps);
+  const int grid = (int)std::min<long long>(ctx->emit_grid, ctas);
+  void* params[] = {&a, &ctx->h_tables};
+  const int big = a.n <= ctx->num_sms ? 1 : 0;
+  VOX_CUDA(ctx, cudaLaunchKernel(ks.list[gm][big], dim3(a.n), dim3(ks.list_threads[big]), params,
+                                 (size_t)ks.list_smem[gm], stream),
+           "cudaLaunchKernel(lists)");
+  cudaLaunchAttribute attr;
+  std::memset(&attr, 0, sizeof attr);
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(ks.emit_threads);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  VOX_CUDA(ctx, cudaLaunchKernelExC(&cfg, ks.emit[ctx->cfg.layout], params), "cudaLaunchKernelExC(emission)");
+  return VOX_OK;
+}
+
 // Issues one fused batch launch with the context's tuning on `stream`; the scratch of the
 // schedule (a.state, or a.scratch + a.counts) is already in `a`.
 int issue_batch(vox_ctx* ctx, MeshArgs& a, int gm, bool host_out, cudaStream_t stream) {
+  if (use_lists(ctx, gm, host_out)) return issue_lists(ctx, a, gm, stream);
   const int layout = ctx->cfg.layout;
   const int threads = ctx->ks->threads[ctx->topt];
   const int smem = ctx->ks->smem_total(layout, threads, host_out ? kStageSingle : ctx->stage_faces);
@@ -364,8 +426,9 @@ int issue_batch(vox_ctx* ctx, MeshArgs& a, int gm, bool host_out, cudaStream_t s
   if (ctx->schedule == VOX_SCHEDULE_PHASED || ctx->schedule == VOX_SCHEDULE_OVERLAP) {
     const bool phased = ctx->schedule == VOX_SCHEDULE_PHASED;
     const void* fn = (phased ? ctx->ks->phased : ctx->ks->overlap)[gm][layout][ctx->topt];
-    const int grid = std::max(1, std::min(a.n, host_out ? ctx->host_grid[gm]
-                                             : phased ? ctx->phased_grid[gm] : ctx->overlap_grid[gm]));
+    const int most = host_out ? ctx->host_grid[gm]
+                     : phased ? ctx->phased_grid[gm] : ctx->overlap_grid[gm];
+    const int grid = std::max(1, std::min(a.n, most));
     // emission items per chunk: one for small chunks unless there are fewer chunks than
     // CTAs; chunks of 32^3 and up (whose emission dwarfs an item's reload) split until
     // there are about eight items per CTA, which evens out the last wave
@@ -518,7 +581,7 @@ int batch_launch(vox_ctx* ctx, MeshArgs& a, int gm, bool host_out = false) {
   }
   const int slab = slab_of(ctx, a.n);
   if (ctx->schedule != VOX_SCHEDULE_LOOKBACK) {  // the spill slots of phases A and C
-    if ((st = ensure_scratch(ctx, (size_t)slab)) != VOX_OK) return st;
+    if ((st = ensure_scratch(ctx, (size_t)slab, slot_bytes(ctx, gm, host_out))) != VOX_OK) return st;
     a.scratch = ctx->d_scratch;
     a.counts = ctx->d_counts;
   }
@@ -622,6 +685,16 @@ int vox_ctx_create(const vox_config* cfg, void* stream, vox_ctx** out) {
   if (cudaMalloc(&ctx->d_tables, sizeof(TablesDev)) != cudaSuccess) return cleanup(VOX_ERR_OOM);
   if (cudaMemcpy(ctx->d_tables, &tab, sizeof tab, cudaMemcpyHostToDevice) != cudaSuccess)
     return cleanup(VOX_ERR_CUDA);
+  if (ctx->gm == GM_HEIGHT) {
+    float2 grad2[kGrad2];
+    for (int i = 0; i < kGrad2; ++i) {
+      const float* gr = tab.grad[tab.perm[tab.perm[i]] & 15];
+      grad2[i] = float2{gr[0], gr[1]};
+    }
+    if (cudaMalloc(&ctx->d_grad2, sizeof grad2) != cudaSuccess) return cleanup(VOX_ERR_OOM);
+    if (cudaMemcpy(ctx->d_grad2, grad2, sizeof grad2, cudaMemcpyHostToDevice) != cudaSuccess)
+      return cleanup(VOX_ERR_CUDA);
+  }
   if (cudaMalloc(&ctx->d_ctl, sizeof(BatchCtl)) != cudaSuccess) return cleanup(VOX_ERR_OOM);
   if (cudaMemset(ctx->d_ctl, 0, sizeof(BatchCtl)) != cudaSuccess) return cleanup(VOX_ERR_CUDA);
   if (cudaMallocHost(&ctx->h_ctl, sizeof(BatchCtl)) != cudaSuccess) return cleanup(VOX_ERR_OOM);
@@ -647,6 +720,18 @@ int vox_ctx_create(const vox_config* cfg, void* stream, vox_ctx** out) {
         (ctx->ks->generate_planes[gm] &&
          (st = prepare_kernel(ctx, ctx->ks->generate_planes[gm], gsmem)) != VOX_OK))
       return cleanup(st);
+  for (int gm = 0; gm < 4; ++gm)
+    for (int t = 0; t < 2; ++t)
+      if (ctx->ks->list[gm][t] &&
+          (st = prepare_kernel(ctx, ctx->ks->list[gm][t], ctx->ks->list_smem[gm])) != VOX_OK)
+        return cleanup(st);
+  {
+    int per_sm = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, ctx->ks->emit[layout], ctx->ks->emit_threads, 0);
+    if (e != cudaSuccess) return cleanup(cuda_fail(ctx, e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor"));
+    ctx->emit_grid = std::max(1, per_sm) * ctx->num_sms;
+  }
   if (apply_tuning(ctx, default_topt(cfg->chunk_size), kStageSingle, 0, kDefaultSchedule, 0, 0) != VOX_OK &&
       (st = apply_tuning(ctx, 0, 0, 0, kDefaultSchedule, 0, 0)) != VOX_OK)  // no room to stage
     return cleanup(st);
@@ -661,6 +746,7 @@ int vox_ctx_destroy(vox_ctx* ctx) {
   if (!ctx) return VOX_OK;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   cudaFree(ctx->d_tables);
+  cudaFree(ctx->d_grad2);
   cudaFree(ctx->d_ctl);
   cudaFree(ctx->d_state);
   cudaFree(ctx->d_scratch);
@@ -694,6 +780,8 @@ static int sync_locked(vox_ctx* ctx) {
   ctx->h_ctl->err = 0;
   if (err & ERR_TIMEOUT) {
     ctx->h_ctl->next = 0;
+    ctx->h_ctl->next_scan = 0;
+    ctx->h_ctl->done = 0;
     ctx->h_ctl->bar_count = 0;
     ctx->h_ctl->epoch += 1;
   }
@@ -1157,6 +1245,11 @@ int vox_autotune(vox_ctx* ctx, const vox_chunk_coord* d_coords, const uint8_t* d
       for (int s : stages) {
         int full_grid = 0;
         for (int c : ctas) {
+          // the list launches have shapes of their own: one candidate, with the default shape
+          // (which launches that write host memory use)
+          if (p == VOX_SCHEDULE_OVERLAP && ctx->gm != GM_BERNOULLI &&
+              (t != default_topt(ctx->cfg.chunk_size) || s != kStageSingle || c != 0))
+            continue;
           if (apply_tuning(ctx, t, s, c, p, 0, 0) != VOX_OK) continue;
           const int g = p == VOX_SCHEDULE_PHASED    ? ctx->phased_grid[ctx->gm]
                         : p == VOX_SCHEDULE_OVERLAP ? ctx->overlap_grid[ctx->gm]
@@ -1258,14 +1351,15 @@ int vox_graph_capture(vox_ctx* ctx, const vox_chunk_coord* d_coords, const uint8
   const int slab = slab_of(ctx, n);
   g->launches = (n + slab - 1) / slab;
   if (g->schedule != VOX_SCHEDULE_LOOKBACK) {
-    if ((e = cudaMalloc(&g->d_scratch, (size_t)slab * (size_t)ctx->ks->spill_bytes)) != cudaSuccess ||
+    const size_t slot = slot_bytes(ctx, ctx->halo_staging ? GM_OCC : ctx->gm, false);
+    if ((e = cudaMalloc(&g->d_scratch, (size_t)slab * slot)) != cudaSuccess ||
         (e = cudaMalloc(&g->d_counts, (size_t)slab * sizeof(uint32_t))) != cudaSuccess)
       return bail(cuda_fail(ctx, e, "cudaMalloc(graph scratch)"));
     a.scratch = g->d_scratch;
     a.counts = g->d_counts;
   }
   if (g->schedule != VOX_SCHEDULE_PHASED) {
-    g->state_bytes = (size_t)slab * sizeof(unsigned long long);
+    g->state_bytes = (size_t)state_words((size_t)slab) * sizeof(unsigned long long);
     if ((e = cudaMalloc(&g->d_state, g->state_bytes)) != cudaSuccess ||
         (e = cudaMemsetAsync(g->d_state, 0, g->state_bytes, ctx->stream)) != cudaSuccess)
       return bail(cuda_fail(ctx, e, "cudaMalloc(graph state)"));

@@ -78,20 +78,22 @@ __host__ __device__ constexpr int dens_max_corners() { return N <= 8 ? 128 : (N 
 // corner-table base, corners along y and along z), DensAxis axes[octave][axis][N + 2],
 // then the corner-pair records: record i holds the gradients of corner i and of corner i + 1
 // (its +z neighbour on the lattice) as {gx_i, gx_i+1, gy_i, gy_i+1} and {gz_i, gz_i+1}; then
-// the coarse samples and the cells of 8^3 voxels they decide (dens_cells): per (y, z) cell
-// row and 32-bit row word, the solid bits and the bits still to be evaluated, the list of
+// the coarse samples and the cells of 8 x 4 x 8 voxels they decide (gen_density): per (y, z)
+// cell row and 32-bit row word, the solid bits and the bits still to be evaluated, the list of
 // the words with any such bits, and its length.
 template <int N>
 struct DensPlan {
-  static constexpr int kCells = N / 8;                       // cells along an axis
-  static constexpr int kPts = kCells + 1;                    // coarse samples along an axis
+  static constexpr int kCells = N / 8;                       // cells along x and along z
+  static constexpr int kCellsY = N / 4;                      // cells along y
+  static constexpr int kPts = kCells + 1;                    // coarse samples along x and z
+  static constexpr int kPtsY = kCellsY + 1;
   static constexpr int kSegs = N > 32 ? N / 32 : 1;          // 32-bit words per row
-  static constexpr int kWords = kCells * kCells * kSegs;     // row words over all (y, z) cells
+  static constexpr int kWords = kCellsY * kCells * kSegs;    // row words over all (y, z) cells
   static constexpr int kAxes = 64;
   static constexpr int kPairXY = kAxes + kDensMaxOct * 3 * (N + 2) * 16;
   static constexpr int kPairZ = kPairXY + dens_max_corners<N>() * 16;
   static constexpr int kCoarse = kPairZ + dens_max_corners<N>() * 8;
-  static constexpr int kKnown = kCoarse + align16(kPts * kPts * kPts * 4);
+  static constexpr int kKnown = kCoarse + align16(kPtsY * kPts * kPts * 4);
   static constexpr int kMixed = kKnown + align16(kWords * 4);
   static constexpr int kList = kMixed + align16(kWords * 4);  // [0]: length, then word indices
   static constexpr int kBytes = kList + align16((kWords + 1) * 4);
@@ -343,8 +345,10 @@ struct ChunkSmem {
   int* hhdr;        // heightmap corner tables: per octave base, corners along z, first x, first z;
                     // [4 * kOctGroup] = corner count, or -1 when the tables are not used
   float2* hcorner;  // heightmap corner gradient coefficients (gx, gy)
+  const float2* grad2;  // gradients of the hashed corners (512), or unused
 
-  __device__ void carve(unsigned char* base) {
+  __device__ void carve(unsigned char* base) { carve(base, SmemPlan<N, LAYOUT>::list_bytes(blockDim.x)); }
+  __device__ void carve(unsigned char* base, int list_bytes) {
     using P = SmemPlan<N, LAYOUT>;
     unsigned char* q = base;
     tab = reinterpret_cast<TablesDev*>(q);
@@ -362,7 +366,12 @@ struct ChunkSmem {
     misc = reinterpret_cast<int*>(q);
     q += P::kMisc;
     lists = reinterpret_cast<uint32_t*>(q);
-    q += P::list_bytes(blockDim.x);
+    q += list_bytes;
+    scratch_at(q);
+  }
+  // The staging area, and the generation scratch in the same place, at q.
+  __device__ void scratch_at(unsigned char* q) {
+    using P = SmemPlan<N, LAYOUT>;
     stage = q;
     colk = reinterpret_cast<int*>(q);
     ax = reinterpret_cast<AxisX*>(q + P::kColK);
@@ -378,6 +387,14 @@ __device__ __forceinline__ void load_tables(ChunkSmem<N, LAYOUT>& s, const Table
   const uint32_t* src = reinterpret_cast<const uint32_t*>(g);
   uint32_t* dst = reinterpret_cast<uint32_t*>(s.tab);
   for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+}
+
+// The hashed gradient table (MeshArgs::grad2, kGrad2 entries) into shared memory at dst.
+template <int T, int N, int LAYOUT>
+__device__ __forceinline__ void load_grad2(ChunkSmem<N, LAYOUT>& s, float2* dst, const float2* src) {
+  const float4* from = reinterpret_cast<const float4*>(src);
+  for (int i = threadIdx.x; i < kGrad2 / 2; i += T) reinterpret_cast<float4*>(dst)[i] = __ldg(from + i);
+  s.grad2 = dst;
 }
 
 // Write one ballot word for the element run [e0, e0 + 32) of a row-major bit array
@@ -421,8 +438,9 @@ __device__ __forceinline__ void halo_coord(int h, int a, int b, int& x, int& y, 
 // fBm of the per-column path (d_noise2_axes with the lattice data of this column), then
 // k = ceil(base + amp * fbm) - oy clamped to [-1, N + 1] (-1 for NaN), so that voxel
 // (x, y, z) is solid iff y < k. The same operations, in the same order, as the shared-table
-// path below and as the oracle.
-template <int N, int LAYOUT>
+// path below and as the oracle. With kHashed, s.grad2 holds the gradients of the hashed corners
+// (entry A = gradient of p[p[A]]), so a corner is one load instead of a chain of three.
+template <int N, bool kHashed = false, int LAYOUT>
 __device__ __forceinline__ int column_k(const ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox,
                                         int oy, int oz, int x, int z) {
   const uint8_t* p = s.tab->perm;
@@ -442,7 +460,17 @@ __device__ __forceinline__ int column_k(const ChunkSmem<N, LAYOUT>& s, const Gen
     az.fr = cz - flz;
     az.v = d_fade(az.fr);
     az.pad = 0;
-    sum = sum + amp * d_noise2_axes(p, gt, ax, az);
+    if (kHashed) {
+      const float2* A = s.grad2 + ax.px + az.y;
+      const float2* B = s.grad2 + ax.px1 + az.y;
+      const float2 g00 = A[0], g01 = A[1], g10 = B[0], g11 = B[1];
+      const float x0 = ax.fr, y0 = az.fr, x1 = x0 - 1.0f, y1 = y0 - 1.0f;
+      const float l0 = d_lerp(ax.u, g00.x * x0 + g00.y * y0, g10.x * x1 + g10.y * y0);
+      const float l1 = d_lerp(ax.u, g01.x * x0 + g01.y * y1, g11.x * x1 + g11.y * y1);
+      sum = sum + amp * d_lerp(az.v, l0, l1);
+    } else {
+      sum = sum + amp * d_noise2_axes(p, gt, ax, az);
+    }
     f = f * g.lac;
     amp = amp * g.gain;
   }
@@ -464,7 +492,7 @@ __device__ __forceinline__ int column_k(const ChunkSmem<N, LAYOUT>& s, const Gen
 // so generation needs no CTA barrier before the row ballots. The shared-table path (larger
 // chunks): the lattice data and corner tables are built once per octave in shared memory,
 // every thread accumulates its columns, and the thresholds go through s.colk.
-template <int N, int LAYOUT, int T>
+template <int N, int LAYOUT, int T, bool kHashed>
 __device__ void gen_heightmap(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, int oy, int oz,
                               unsigned halo_mask, bool with_halo) {
   using RowT = typename Shape<N>::RowT;
@@ -621,86 +649,83 @@ __device__ void gen_heightmap(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, 
     }
     __syncthreads();
   }  // !direct
-  // Rows from the column thresholds, one warp task per group of columns: the own rows of
-  // a group of z values (and their -y / +y halo rows), or one lateral halo strip. Lanes
-  // hold one column's threshold k each; rows below the group's smallest k are full, rows
-  // at or above its largest k are empty, and the rows in between are ballots of y < k.
+  // Rows from the column thresholds, one warp task per 32 columns: the own columns of a group of
+  // z values, or the columns of the lateral halo strips (for N < 32 several side by side).
+  // Lanes hold one column's threshold k each. Row y of the task is the ballot of y < k: full
+  // below the task's smallest k, empty from its largest on, so only the rows in between are
+  // voted on; lane y keeps row y, and one store per lane writes the rows.
   {
-    constexpr int G = N >= 32 ? 1 : 32 / N;  // z values per own-row task
     constexpr int S = N > 32 ? N / 32 : 1;   // 32-bit words per row
     constexpr int LW = N >= 32 ? 32 : N;     // lanes per row word
+    constexpr int G = 32 / LW;               // z values per own task
+    constexpr int HP = G < 4 ? G : 4;        // halo strips per halo task
     constexpr int W = Shape<N>::W;
+    constexpr int YP = N > 32 ? N / 32 : 1;  // rows a lane keeps
     constexpr uint32_t kWordFull = N >= 32 ? 0xFFFFFFFFu : ((1u << (N & 31)) - 1u);
     constexpr int kOwnTasks = (N / G) * S;
+    const int tasks = kOwnTasks + (with_halo ? (4 / HP) * S : 0);
     const int lane = t & 31, warp = t >> 5;
     constexpr int nwarps = T / 32;
     uint32_t* occw = reinterpret_cast<uint32_t*>(s.occ);
     uint32_t* halow = reinterpret_cast<uint32_t*>(s.halo);
     const int sub = lane / LW, b = lane % LW;  // row word group and bit of this lane
-    for (int task = warp; task < kOwnTasks + 4 * S; task += nwarps) {
+    const bool vertical = with_halo && (halo_mask >> 4) != 0u;
+    for (int task = warp; task < tasks; task += nwarps) {
       const bool own = task < kOwnTasks;
-      const int h = own ? -1 : (task - kOwnTasks) / S;
       const int seg = own ? task % S : (task - kOwnTasks) % S;
       const int xb = seg * 32 + b;  // bit position within the row
-      int k;
-      bool active = true;  // lanes past the end of a short halo strip hold no column
-      uint32_t* base;      // word of row a of the task's first row group: base[a * rstride]
-      int rstride;
-      if (own) {
-        const int z = (task / S) * G + sub;
-        k = direct ? column_k<N, LAYOUT>(s, g, ox, oy, oz, xb, z) : s.colk[(z + 1) * side + xb + 1];
-        base = occw + (task / S) * G * W + seg;
-        rstride = N * W;
-      } else {
-        // lateral halo h: row a = y, bit = position along the strip
-        const int c = sub == 0 ? xb : -1;
-        active = c >= 0;
-        const bool used = ((halo_mask >> h) & 1u) && with_halo;
-        if (c < 0 || !used) {
-          k = -1;
-        } else if (direct) {
-          const int hx = h == 0 ? -1 : (h == 1 ? N : c), hz = h == 2 ? -1 : (h == 3 ? N : c);
-          k = column_k<N, LAYOUT>(s, g, ox, oy, oz, hx, hz);
-        } else if (h == 0) {
-          k = s.colk[(c + 1) * side];
-        } else if (h == 1) {
-          k = s.colk[(c + 1) * side + N + 1];
-        } else if (h == 2) {
-          k = s.colk[c + 1];
-        } else {
-          k = s.colk[(N + 1) * side + c + 1];
-        }
-        base = halow + h * N * W + seg;
-        rstride = W;
+      const int z0 = (task / S) * G, h0 = own ? 0 : ((task - kOwnTasks) / S) * HP;
+      int x = xb, z = z0 + sub;
+      bool used = true;
+      if (!own) {
+        const int h = h0 + (sub < HP ? sub : HP - 1);
+        used = ((halo_mask >> h) & 1u) != 0u;
+        x = h == 0 ? -1 : (h == 1 ? N : xb);
+        z = h == 2 ? -1 : (h == 3 ? N : xb);
       }
-      const int kmin = __reduce_min_sync(0xffffffffu, active ? k : N + 1);
-      const int kmax = __reduce_max_sync(0xffffffffu, active ? k : -1);
-      // trivial rows (own tasks: G rows of each y; halo tasks: one row of each y)
-      const int gw = own ? G : 1;
-      for (int j = lane; j < N * gw; j += 32) {
-        const int y = j / gw, zz = j % gw;
-        base[y * rstride + zz * W] = y < kmin ? kWordFull : 0u;
+      int k = -1;
+      if (used) {
+        k = direct ? column_k<N, kHashed>(s, g, ox, oy, oz, x, z) : s.colk[(z + 1) * side + x + 1];
       }
-      __syncwarp();
-      const int y0 = kmin < 0 ? 0 : kmin, y1 = kmax > N ? N : kmax;
-      for (int y = y0; y < y1; ++y) {
+      const int kmin = __reduce_min_sync(0xffffffffu, k), kmax = __reduce_max_sync(0xffffffffu, k);
+      uint32_t keep[YP];
+#pragma unroll
+      for (int j = 0; j < YP; ++j) keep[j] = lane + 32 * j < kmin ? 0xFFFFFFFFu : 0u;
+      for (int y = kmin < 0 ? 0 : kmin; y < (kmax > N ? N : kmax); ++y) {
         const uint32_t bal = __ballot_sync(0xffffffffu, y < k);
-        if (b == 0 && (own || sub == 0))
-          base[y * rstride + sub * W] = N >= 32 ? bal : ((bal >> lane) & kWordFull);
+#pragma unroll
+        for (int j = 0; j < YP; ++j)
+          if (lane + 32 * j == y) keep[j] = bal;
       }
-      if (own) {
-        // -y and +y halo rows of these z values (bits x): y = -1 and y = N
-        const bool use4 = with_halo && ((halo_mask >> 4) & 1u);
-        const bool use5 = with_halo && ((halo_mask >> 5) & 1u);
-        const uint32_t b4 = __ballot_sync(0xffffffffu, use4 && -1 < k);
-        const uint32_t b5 = __ballot_sync(0xffffffffu, use5 && N < k);
-        if (b == 0 && with_halo) {
-          const int z = (task / S) * G + sub;
-          halow[(4 * N + z) * W + seg] = N >= 32 ? b4 : ((b4 >> lane) & kWordFull);
-          halow[(5 * N + z) * W + seg] = N >= 32 ? b5 : ((b5 >> lane) & kWordFull);
+#pragma unroll
+      for (int j = 0; j < YP; ++j) {
+        const int y = lane + 32 * j;
+        if (y >= N) continue;
+        if (!own) {
+#pragma unroll
+          for (int q = 0; q < HP; ++q)
+            halow[((h0 + q) * N + y) * W + seg] = (keep[j] >> ((q * LW) & 31)) & kWordFull;
+        } else if (N == 16) {
+          *reinterpret_cast<uint2*>(occw + y * N + z0) = make_uint2(keep[j] & 0xFFFFu, keep[j] >> 16);
+        } else if (N == 8) {
+          *reinterpret_cast<uint4*>(occw + y * N + z0) = make_uint4(
+              keep[j] & 0xFFu, (keep[j] >> 8) & 0xFFu, (keep[j] >> 16) & 0xFFu, keep[j] >> 24);
+        } else {
+          occw[(y * N + z0) * W + seg] = keep[j];
         }
       }
-      __syncwarp();
+      if (own && with_halo) {
+        // -y and +y halo rows of these z values (bits x): y = -1 and y = N
+        uint32_t b4 = 0u, b5 = 0u;
+        if (vertical) {
+          b4 = __ballot_sync(0xffffffffu, ((halo_mask >> 4) & 1u) && -1 < k);
+          b5 = __ballot_sync(0xffffffffu, ((halo_mask >> 5) & 1u) && N < k);
+        }
+        if (b == 0) {
+          halow[(4 * N + z) * W + seg] = (b4 >> lane) & kWordFull;
+          halow[(5 * N + z) * W + seg] = (b5 >> lane) & kWordFull;
+        }
+      }
     }
   }
   __syncthreads();
@@ -872,9 +897,9 @@ __device__ __forceinline__ float dens_value_tab(const ChunkSmem<N, LAYOUT>& s, c
 // second derivative (per squared cell) below 12.1 for every choice of gradients (a test
 // computes both from the formulas). So the density, the fBm minus a term linear in y, stays
 // within 1.037 * sum|amp| of that term, and inside a cell of voxels of edge h it stays within
-// `slack` = 3 axes * 13/8 * sum |amp| (h f)^2 of the range of its values at the cell's eight
+// `slack` = 13/8 * sum |amp| f^2 (h^2 + h^2 + hy^2) of the range of its values at the cell's eight
 // corners (trilinear interpolation error). A cell whose corner densities all exceed the slack
-// with one sign therefore needs no evaluation. `err` covers the rounding of the computed values
+// with one sign therefore needs no evaluation (the cells are h by h, and hy along y). `err` covers the rounding of the computed values
 // against exact arithmetic: coordinates are off by up to 2^-24 of their size, which moves a
 // value by less than 2e-6 * |c| (the slope of the noise is below 5 a cell on each axis); the
 // arithmetic of one value rounds to less than 4e-5; the height term and the sum to less than
@@ -886,15 +911,16 @@ struct DensBounds {
   float slack;  // a cell with corner densities beyond +-slack is known; infinite: none is
 };
 template <int N>
-__device__ __forceinline__ DensBounds dens_bounds(const GenDev& g, int ox, int oy, int oz, float h) {
+__device__ __forceinline__ DensBounds dens_bounds(const GenDev& g, int ox, int oy, int oz, float h,
+                                                  float hy) {
   constexpr int kLim = (1 << 24) - 256;
   const bool exact = ox > -kLim && ox < kLim && oy > -kLim && oy < kLim && oz > -kLim && oz < kLim;
   const float cm = (float)(max(max(abs(ox), abs(oy)), abs(oz)) + N + 1);
   float A = 0.0f, S = 0.0f, err = 0.0f, f = g.freq, amp = 1.0f;
   for (int o = 0; o < g.octaves; ++o) {
-    const float a = fabsf(amp), hf = h * f;
+    const float a = fabsf(amp);
     A = A + a;
-    S = S + a * (hf * hf);
+    S = S + a * (f * f);
     err = err + a * (2e-6f * (cm * fabsf(f)) + 4e-5f);
     f = f * g.lac;
     amp = amp * g.gain;
@@ -907,7 +933,7 @@ __device__ __forceinline__ DensBounds dens_bounds(const GenDev& g, int ox, int o
   r.known = -1;
   if (exact && t0 > b && t1 > b) r.known = g.solid_below_zero ? 1 : 0;    // every d < 0
   if (exact && t0 < -b && t1 < -b) r.known = g.solid_below_zero ? 0 : 1;  // every d > 0
-  const float slack = 4.875f * S + 2.0f * err;
+  const float slack = 1.625f * (2.0f * h * h + hy * hy) * S + 2.0f * err;
   r.slack = exact && slack < A ? slack : __int_as_float(0x7f800000);
   return r;
 }
@@ -991,9 +1017,10 @@ __device__ __forceinline__ uint32_t dens_block_z(const ChunkSmem<N, LAYOUT>& s, 
   return keep;
 }
 
-// The same with the samples along y, for the lateral halo planes (lane: a position along the
-// plane, x or z; the other coordinate fixed): lane i of the first kDensB gets the ballot of
+// The same with kDensY samples along y, for the lateral halo planes (lane: a position along the
+// plane, x or z; the other coordinate fixed): lane i of the first kDensY gets the ballot of
 // y = ys + i. The records are held with g.x * x and g.z * z.
+constexpr int kDensY = 4;
 template <int N, int LAYOUT>
 __device__ __forceinline__ uint32_t dens_block_y(const ChunkSmem<N, LAYOUT>& s, const GenDev& g, int oy,
                                                  int x, int ys, int z) {
@@ -1002,9 +1029,9 @@ __device__ __forceinline__ uint32_t dens_block_y(const ChunkSmem<N, LAYOUT>& s, 
   const DensAxis* axes = reinterpret_cast<const DensAxis*>(s.stage + P::kAxes);
   const ulonglong2* pair_xy = reinterpret_cast<const ulonglong2*>(s.stage + P::kPairXY);
   const f2_t* pair_z = reinterpret_cast<const f2_t*>(s.stage + P::kPairZ);
-  float sum[kDensB];
+  float sum[kDensY];
 #pragma unroll
-  for (int i = 0; i < kDensB; ++i) sum[i] = 0.0f;
+  for (int i = 0; i < kDensY; ++i) sum[i] = 0.0f;
   float amp = 1.0f;
 #pragma unroll 1
   for (int o = 0; o < g.octaves; ++o) {
@@ -1019,7 +1046,7 @@ __device__ __forceinline__ uint32_t dens_block_y(const ChunkSmem<N, LAYOUT>& s, 
     f2_t px00 = 0, px10 = 0, px01 = 0, px11 = 0;  // {gx * x}
     f2_t pz00 = 0, pz10 = 0, pz01 = 0, pz11 = 0;  // {gz * zf, gz' * (zf - 1)}
 #pragma unroll
-    for (int i = 0; i < kDensB; ++i) {
+    for (int i = 0; i < kDensY; ++i) {
       const DensAxis ay = ya[i];  // the same in every lane
       if (ay.ci != cur) {
         cur = ay.ci;
@@ -1050,7 +1077,7 @@ __device__ __forceinline__ uint32_t dens_block_y(const ChunkSmem<N, LAYOUT>& s, 
   const int lane = threadIdx.x & 31;
   uint32_t keep = 0u;
 #pragma unroll
-  for (int i = 0; i < kDensB; ++i) {
+  for (int i = 0; i < kDensY; ++i) {
     const float d = sum[i] - ((float)(oy + ys + i) - g.y_ref) * g.y_scale;
     const uint32_t b = __ballot_sync(0xffffffffu, g.solid_below_zero ? (d < 0.0f) : (d > 0.0f));
     if (lane == i) keep = b;
@@ -1061,10 +1088,12 @@ __device__ __forceinline__ uint32_t dens_block_y(const ChunkSmem<N, LAYOUT>& s, 
 // A density chunk and its halo planes, or false (without a barrier) when the configuration is
 // beyond the lattice tables (the caller then evaluates sample by sample). Chunks whose bounds
 // decide them (dens_bounds) cost neither tables nor noise. Else the density is sampled on a
-// coarse grid (spacing 8: points 0, 8, ..., N; with halos -1, 7, ..., N, so that the planes at
-// -1 and N are inside too, one spacing of 9), which decides most cells of 8^3 voxels; the rest
-// are evaluated, a warp taking one row word at 8 consecutive z (dens_block_z), and the
-// undecided parts of the lateral planes 8 rows at a time (dens_block_y).
+// coarse grid, which decides most cells of 8 x 4 x 8 voxels (spacing 8 along x and z: points 0,
+// 8, ..., N, with halos -1, 7, ..., N, so that the planes at -1 and N are inside too, one spacing
+// of 9; along y the same with 4). The rest are evaluated, a warp taking one row word at 8
+// consecutive z (dens_block_z), and the undecided parts of the lateral planes 4 rows at a time
+// (dens_block_y). Work goes by rows, so cells flat in y leave less to evaluate: with cells of
+// 8^3 a cave chunk at the surface evaluates 37 row words of 128, with 8 x 4 x 8 about 25.
 // On the 4096-chunk 32^3 cave terrain (3 octaves at 1/96; 55 % of the chunks are decided by
 // their bounds, about 9 % of all samples are evaluated) vox_generate went from 610 us, bound by
 // the FP32 pipe with every sample evaluated and x as the inner axis, to 103 us; the fused
@@ -1078,11 +1107,11 @@ __device__ bool gen_density(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, in
   constexpr int LX = N < 32 ? N : 32;       // lanes along a row word
   constexpr int kSub = 32 / LX;             // y rows a warp evaluates side by side
   constexpr uint32_t kWordFull = N >= 32 ? 0xFFFFFFFFu : ((1u << (N & 31)) - 1u);
-  constexpr int C = P::kCells;
+  constexpr int C = P::kCells, CY = P::kCellsY;
   const int t = threadIdx.x;
   uint32_t* occw = reinterpret_cast<uint32_t*>(s.occ);
   uint32_t* halow = reinterpret_cast<uint32_t*>(s.halo);
-  const DensBounds bd = dens_bounds<N>(g, ox, oy, oz, with_halo ? 9.0f : 8.0f);
+  const DensBounds bd = dens_bounds<N>(g, ox, oy, oz, with_halo ? 9.0f : 8.0f, with_halo ? 5.0f : 4.0f);
   if (bd.known >= 0) {
     const RowT v = bd.known ? full_row<N>() : (RowT)0;
     for (int i = t; i < N * N; i += T) s.occ[i] = v;
@@ -1099,11 +1128,12 @@ __device__ bool gen_density(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, in
   const bool use_coarse = bd.slack < 3.0e38f;
   if (t == 0) list[0] = 0;
   if (use_coarse) {
-    constexpr int Q = P::kPts;
-    for (int i = t; i < Q * Q * Q; i += T) {
+    constexpr int Q = P::kPts, QY = P::kPtsY;
+    for (int i = t; i < QY * Q * Q; i += T) {
       const int px = i % Q, pz = (i / Q) % Q, py = i / (Q * Q);
       auto at = [&](int p) { return with_halo ? (p == C ? N : 8 * p - 1) : 8 * p; };
-      coarse[i] = dens_value_tab<N, LAYOUT>(s, g, at(px), at(py), at(pz), oy);
+      const int y = with_halo ? (py == CY ? N : 4 * py - 1) : 4 * py;
+      coarse[i] = dens_value_tab<N, LAYOUT>(s, g, at(px), y, at(pz), oy);
     }
   }
   __syncthreads();
@@ -1140,22 +1170,22 @@ __device__ bool gen_density(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, in
   // decided cell rows: their words at every voxel row
   for (int i = t; i < N * N * W; i += T) {
     const int seg = i % W, z = (i / W) % N, y = i / (W * N);
-    const int c = ((y >> 3) * C + (z >> 3)) * P::kSegs + seg;
+    const int c = ((y >> 2) * C + (z >> 3)) * P::kSegs + seg;
     if (mixed[c] == 0u) occw[i] = known[c];
   }
   // Work items of a warp: the undecided row words (kSub rows y, 8 z each), then the lateral
-  // halo planes (kPl planes side by side, 8 rows y), then the -y and +y planes (8 rows z).
+  // halo planes (kPl planes side by side, 4 rows y), then the -y and +y planes (8 rows z).
   constexpr int kPl = kSub < 2 ? 1 : 2;
-  constexpr int kPerCell = 8 / kSub;
+  constexpr int kPerCell = 4 / kSub;
   const int own = list[0] * kPerCell;
-  const int lateral = with_halo ? (4 / kPl) * C * P::kSegs : 0;
+  const int lateral = with_halo ? (4 / kPl) * CY * P::kSegs : 0;
   const int vertical = with_halo ? 2 * C * P::kSegs : 0;
   const int lane = t & 31, lx = lane % LX, sub = lane / LX;
   for (int it = t >> 5; it < own + lateral + vertical; it += T / 32) {
     if (it < own) {
       const int c = list[1 + it / kPerCell];
       const int seg = c % P::kSegs, cz = (c / P::kSegs) % C, cy = c / (P::kSegs * C);
-      const int y = cy * 8 + (it % kPerCell) * kSub, zs = cz * 8;
+      const int y = cy * 4 + (it % kPerCell) * kSub, zs = cz * 8;
       const uint32_t b = dens_block_z<N, LAYOUT>(s, g, oy, seg * 32 + lx, y + sub, zs);
       if (lane < kDensB) {
 #pragma unroll
@@ -1164,9 +1194,9 @@ __device__ bool gen_density(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, in
       }
     } else if (it < own + lateral) {
       const int k = it - own;
-      const int seg = k % P::kSegs, cy = (k / P::kSegs) % C, h0 = (k / (P::kSegs * C)) * kPl;
+      const int seg = k % P::kSegs, cy = (k / P::kSegs) % CY, h0 = (k / (P::kSegs * CY)) * kPl;
       const int pl = sub < kPl ? sub : kPl - 1;  // 8^3 chunks: the lanes past two planes repeat
-      const int h = h0 + pl, ys = cy * 8;
+      const int h = h0 + pl, ys = cy * 4;
       // decided bits and undecided bits of this lane's plane word (a decided cell is one byte)
       uint32_t kn = 0u, mi = 0u;
       if (h >= 2) {  // z planes: words along x of the first or last cell row
@@ -1194,7 +1224,7 @@ __device__ bool gen_density(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, in
         for (int q = 0; q < kPl; ++q)
           b |= (__shfl_sync(0xffffffffu, kn, q * LX) & kWordFull) << ((q * LX) & 31);
       }
-      if (lane < kDensB) {
+      if (lane < kDensY) {
 #pragma unroll
         for (int q = 0; q < kPl; ++q)
           halow[((h0 + q) * N + ys + lane) * W + seg] =
@@ -1203,7 +1233,7 @@ __device__ bool gen_density(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, in
     } else {
       const int k = it - own - lateral;
       const int seg = k % P::kSegs, cz = (k / P::kSegs) % C, h = 4 + k / (P::kSegs * C);
-      const int c = ((h == 4 ? 0 : C - 1) * C + cz) * P::kSegs + seg;
+      const int c = ((h == 4 ? 0 : CY - 1) * C + cz) * P::kSegs + seg;
       const bool used = (halo_mask >> h) & 1u;
       uint32_t b = used ? known[c] : 0u;
       if (used && mixed[c] != 0u)
@@ -1217,13 +1247,14 @@ __device__ bool gen_density(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, in
 
 // Fills s.occ (own rows) and, for every set bit of `halo_mask`, the halo rows; the other
 // halo rows are zero (a neighbour that is not loaded counts as air, chunk.rs:102-107).
-template <int N, int GM, int LAYOUT, int T>
+// kHashed: s.grad2 holds the hashed gradients of the heightmap columns (see column_k).
+template <int N, int GM, int LAYOUT, int T, bool kHashed = false>
 __device__ void gen_chunk(ChunkSmem<N, LAYOUT>& s, const GenDev& g, vox_chunk_coord c,
                           long long chunk_index, unsigned halo_mask, bool with_halo) {
   using RowT = typename Shape<N>::RowT;
   const int ox = c.x * N, oy = c.y * N, oz = c.z * N;
   if (GM == GM_HEIGHT) {
-    gen_heightmap<N, LAYOUT, T>(s, g, ox, oy, oz, halo_mask, with_halo);
+    gen_heightmap<N, LAYOUT, T, kHashed>(s, g, ox, oy, oz, halo_mask, with_halo);
     return;
   }
   if (GM == GM_DENSITY) {
@@ -1324,15 +1355,23 @@ __device__ __forceinline__ void row_masks(const ChunkSmem<N, LAYOUT>& s, int y, 
   m[5] = row & ~un;
 }
 
-// Per-row face counts -> exclusive offsets in s.rows[0..R], the ascending list of the
-// rows with faces in s.nz (count in s.misc[0]) and, when they fit, the face voxels in
-// emission order in s.vlist (count in s.misc[1], else -1); returns the chunk's face total.
+// Per-row face counts -> exclusive offsets in s.rows[0..R], the face voxels in emission order
+// in s.vlist when they fit (count in s.misc[1], else -1) and, for sizes whose voxels may not
+// fit, the ascending list of the rows with faces in s.nz (count in s.misc[0], else 0); returns
+// the chunk's face total.
 template <int N, int LAYOUT, int T>
 __device__ uint32_t count_and_scan(ChunkSmem<N, LAYOUT>& s) {
   using RowT = typename Shape<N>::RowT;
   constexpr int RPT = Shape<N>::R / T;
   constexpr int VCap = Shape<N>::VCap;
   static_assert(RPT >= 1 && RPT * T == Shape<N>::R, "rows must split evenly over threads");
+  // One packed sum per thread. Where every voxel fits the list (up to 16^3) the rows are not
+  // listed, and faces (at most 3 N^3 + 6 N^2, below 2^14) and face voxels (at most 2^12) fit 32
+  // bits; else 64 bits hold faces, face voxels and rows with faces, 20 bits each.
+  constexpr bool kSmall = VCap >= N * N * N;
+  using SumT = typename std::conditional<kSmall, uint32_t, unsigned long long>::type;
+  constexpr int kFaceShift = kSmall ? 16 : 40, kVoxShift = kSmall ? 0 : 20;
+  constexpr uint32_t kMask = kSmall ? 0xFFFFu : 0xFFFFFu;
   const int t = threadIdx.x;
   uint32_t cnt[RPT];
   RowT any[RPT];
@@ -1340,58 +1379,64 @@ __device__ uint32_t count_and_scan(ChunkSmem<N, LAYOUT>& s) {
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
     const int r = t * RPT + k;
-    RowT m[6];
-    row_masks<N, LAYOUT>(s, r / N, r % N, m);
     uint32_t c = 0;
+    any[k] = (RowT)0;
+    if (s.occ[r] != (RowT)0) {
+      RowT m[6];
+      row_masks<N, LAYOUT>(s, r / N, r % N, m);
 #pragma unroll
-    for (int d = 0; d < 6; ++d) c += (uint32_t)popc_row(m[d]);
+      for (int d = 0; d < 6; ++d) c += (uint32_t)popc_row(m[d]);
+      any[k] = VCap > 0 ? (m[0] | m[1] | m[2] | m[3] | m[4] | m[5]) : (RowT)0;
+    }
     cnt[k] = c;
-    any[k] = VCap > 0 ? (m[0] | m[1] | m[2] | m[3] | m[4] | m[5]) : (RowT)0;
     local += c;
     if (VCap > 0) vl += (uint32_t)popc_row(any[k]);
     nzl += c != 0u ? 1u : 0u;
   }
-  // Deterministic block scan of (faces << 40 | face voxels << 20 | rows with faces); each
-  // field stays below 2^20 (at most 3N^3 + 6N^2 faces): warp inclusive scan, then a scan
-  // of the warp totals.
+  // Deterministic block scan: warp inclusive scan, then a scan of the warp totals.
   const int lane = t & 31, warp = t >> 5, nwarps = T >> 5;
-  const unsigned long long mine =
-      ((unsigned long long)local << 40) | ((unsigned long long)vl << 20) | nzl;
-  unsigned long long incl = mine;
+  const SumT mine = ((SumT)local << kFaceShift) | ((SumT)vl << kVoxShift) | (kSmall ? (SumT)0 : (SumT)nzl);
+  SumT incl = mine;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, off);
+    const SumT v = __shfl_up_sync(0xffffffffu, incl, off);
     if (lane >= off) incl += v;
   }
-  unsigned long long* wsum = reinterpret_cast<unsigned long long*>(s.stage);  // staging is free
+  SumT* wsum = reinterpret_cast<SumT*>(s.stage);  // staging is free
   if (lane == 31) wsum[warp] = incl;
   __syncthreads();
   // every warp scans the warp totals itself (no second barrier)
-  unsigned long long before = 0, tot = 0;
+  SumT before = 0, tot = 0;
   {
-    const unsigned long long v = lane < nwarps ? wsum[lane] : 0ull;
-    unsigned long long vi = v;
+    const SumT v = lane < nwarps ? wsum[lane] : (SumT)0;
+    SumT vi = v;
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const unsigned long long u = __shfl_up_sync(0xffffffffu, vi, off);
+    for (int off = 1; off < T / 32; off <<= 1) {
+      const SumT u = __shfl_up_sync(0xffffffffu, vi, off);
       if (lane >= off) vi += u;
     }
     before = __shfl_sync(0xffffffffu, vi - v, warp);  // exclusive offset of this warp
     tot = __shfl_sync(0xffffffffu, vi, nwarps - 1);   // chunk totals
   }
-  const unsigned long long excl = before + incl - mine;
-  const uint32_t nvox = (uint32_t)(tot >> 20) & 0xFFFFFu;
+  const SumT excl = before + incl - mine;
+  const uint32_t nvox = (uint32_t)(tot >> kVoxShift) & kMask;
   const bool use_list = VCap > 0 && nvox <= (uint32_t)VCap;
-  uint32_t run = (uint32_t)(excl >> 40);
-  uint32_t vrun = (uint32_t)(excl >> 20) & 0xFFFFFu;
-  uint32_t nzrun = (uint32_t)excl & 0xFFFFFu;
+  uint32_t run = (uint32_t)(excl >> kFaceShift);
+  uint32_t vrun = (uint32_t)(excl >> kVoxShift) & kMask;
+  uint32_t nzrun = (uint32_t)excl & kMask;
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
     const int r = t * RPT + k;
     s.rows[r] = run;
-    if (cnt[k] != 0u) s.nz[nzrun++] = (uint16_t)r;
+    if (!kSmall && cnt[k] != 0u) s.nz[nzrun++] = (uint16_t)r;
     if (VCap > 0 && use_list) {
       RowT u = any[k];
+      if (u == full_row<N>()) {  // a face of every voxel: most rows of the chunk's borders
+#pragma unroll
+        for (int x = 0; x < N; ++x) s.vlist[vrun + x] = (uint16_t)((r << Shape<N>::LOG2N) | x);
+        vrun += N;
+        u = (RowT)0;
+      }
       while (u) {
         const int x = __ffs((uint32_t)u) - 1;
         u &= u - (RowT)1;
@@ -1400,32 +1445,26 @@ __device__ uint32_t count_and_scan(ChunkSmem<N, LAYOUT>& s) {
     }
     run += cnt[k];
   }
-  const uint32_t total = (uint32_t)(tot >> 40);
+  const uint32_t total = (uint32_t)(tot >> kFaceShift);
   if (t == 0) {
     s.rows[Shape<N>::R] = total;
-    s.misc[0] = (int)(tot & 0xFFFFFu);
+    s.misc[0] = kSmall ? 0 : (int)(tot & kMask);
     s.misc[1] = use_list ? (int)nvox : -1;
   }
   __syncthreads();
   return total;
 }
 
-// Decoupled look-back over chunks (warp 0 of the CTA). Returns the exclusive prefix of
-// chunk i. Each poll reads a window of 128 predecessors (4 per lane, coalesced), walks
-// back to the nearest inclusive prefix and sums the aggregates in between. Every wait is
-// bounded (spin_limit polls); on timeout the error bit is set and 0 is used.
+// Decoupled look-back (one warp): the sum of the published values of states 0 .. i - 1. Each
+// poll reads a window of 128 predecessors (4 per lane, coalesced), walks back to the nearest
+// inclusive prefix and sums the aggregates in between. Every wait is bounded (spin_limit
+// polls); on timeout the error bit is set and what was summed so far is returned.
 constexpr int kLookbackWindow = 128;
-// publish_agg = false: chunk i's aggregate is already published (overlap schedule).
-static __device__ unsigned long long lookback(unsigned long long* state, BatchCtl* ctl,
-                                              unsigned epoch, int i, unsigned long long total,
-                                              int spin_limit, bool publish_agg = true) {
+static __device__ unsigned long long lookback_sum(unsigned long long* state, BatchCtl* ctl,
+                                                  unsigned epoch, int i, int spin_limit) {
   const int lane = threadIdx.x & 31;
   unsigned long long excl = 0;
-  if (i == 0) {
-    if (lane == 0) st_relaxed_u64(&state[0], pack_state(epoch, kFlagIncl, total));
-    return 0;
-  }
-  if (lane == 0 && publish_agg) st_relaxed_u64(&state[i], pack_state(epoch, kFlagAgg, total));
+  if (i == 0) return 0;
   const unsigned tag = epoch & 0xFFFFFFu;
   const unsigned long long vmask = (1ull << 38) - 1;
   int j = i - 1;
@@ -1476,6 +1515,18 @@ static __device__ unsigned long long lookback(unsigned long long* state, BatchCt
     if (first_incl < kLookbackWindow) break;
     j -= kLookbackWindow;
   }
+  return excl;
+}
+
+// Look-back over chunks (warp 0 of the CTA): the exclusive prefix of chunk i, whose inclusive
+// prefix is published. publish_agg = false: chunk i's aggregate is already published (overlap
+// schedule).
+static __device__ unsigned long long lookback(unsigned long long* state, BatchCtl* ctl,
+                                              unsigned epoch, int i, unsigned long long total,
+                                              int spin_limit, bool publish_agg = true) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0 && publish_agg && i > 0) st_relaxed_u64(&state[i], pack_state(epoch, kFlagAgg, total));
+  const unsigned long long excl = lookback_sum(state, ctl, epoch, i, spin_limit);
   if (lane == 0) st_relaxed_u64(&state[i], pack_state(epoch, kFlagIncl, excl + total));
   return excl;
 }
@@ -1655,18 +1706,18 @@ __device__ __forceinline__ void flush_warp_lanes(const unsigned char* buf, int s
   }
 }
 
-// A face of a warp's face list: local voxel (x, y, z) and emission direction.
+// A face of a face list: local voxel (x, y, z) and emission direction, a byte each.
 __device__ __forceinline__ uint32_t pack_face(int x, int y, int z, int d) {
-  return (uint32_t)x | ((uint32_t)y << 7) | ((uint32_t)z << 14) | ((uint32_t)d << 21);
+  return (uint32_t)x | ((uint32_t)y << 8) | ((uint32_t)z << 16) | ((uint32_t)d << 24);
 }
 
 // Face compaction of one warp: lane l owns element base + l of the chunk's emission
 // elements, the face voxels of s.vlist (use_list) or else every voxel of the rows with
 // faces (rows nz[], N voxels each); either way the warp's voxels are consecutive in
-// emission order. Each lane lists its voxel's faces in direction order into the warp's
-// face list; returns the warp's face count and, in `first`, the chunk-relative index of
-// the warp's first face (face i of the list has index first + i).
-template <int N, int LAYOUT>
+// emission order. Each lane lists its voxel's faces in direction order; returns the warp's
+// face count and, in `first`, the chunk-relative index of the warp's first face. Face i of
+// the warp (index first + i) goes to list[i], or with kAbsolute to list[first + i].
+template <int N, bool kAbsolute = false, int LAYOUT>
 __device__ __forceinline__ int warp_faces(const ChunkSmem<N, LAYOUT>& s, bool use_list,
                                           int elems, int base, uint32_t* list, uint32_t& first) {
   using RowT = typename Shape<N>::RowT;
@@ -1710,11 +1761,12 @@ __device__ __forceinline__ int warp_faces(const ChunkSmem<N, LAYOUT>& s, bool us
   }
   const int total = __shfl_sync(0xffffffffu, incl, 31);
   first = __shfl_sync(0xffffffffu, mine, 0);  // lane 0's voxel starts the warp's range
-  int pos = incl - cnt;
+  uint32_t* out = list + (incl - cnt) + (kAbsolute ? (int)first : 0);
+  const uint32_t code = pack_face(x, y, z, 0);
   while (bits) {
     const int d = __ffs(bits) - 1;
     bits &= bits - 1u;
-    list[pos++] = pack_face(x, y, z, d);
+    *out++ = code | ((uint32_t)d << 24);
   }
   __syncwarp();
   return total;
@@ -1740,80 +1792,98 @@ __device__ __forceinline__ int emit_elems(const ChunkSmem<N, LAYOUT>& s) {
 template <int LAYOUT>
 __host__ __device__ constexpr unsigned line_faces() { return LAYOUT == VOX_LAYOUT_INSTANCED ? 32u : 16u; }
 
+// Sends one batch of nw faces (lane l < nw holds face first + l of the chunk in q) to global
+// faces g, g + 1, ...: staged in one of the warp's nbuf buffers (`bufs`, buffer index b
+// carried across calls) and sent by a TMA bulk copy, or by coalesced lane stores when
+// lane_flush.
+template <int N, int LAYOUT>
+__device__ __forceinline__ void warp_send_batch(const TablesDev* tab, uint32_t q, int nw, uint32_t first,
+                                                vox_chunk_coord c, unsigned long long g, void* out0,
+                                                void* out1, unsigned char* bufs, int nbuf,
+                                                bool lane_flush, int& b) {
+  constexpr int kBuf = warp_buf_bytes<LAYOUT>();
+  const int lane = threadIdx.x & 31;
+  unsigned char* buf = bufs + b * kBuf;
+  // the copy issued nbuf batches ago read this buffer; wait until it is done reading
+  if (lane == 0) {
+    if (nbuf == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+  }
+  __syncwarp();
+  const int shift = stage_shift<LAYOUT>(g);
+  if (lane < nw) {
+    const int x = q & 255, y = (q >> 8) & 255, z = (q >> 16) & 255, d = q >> 24;
+    stage_face<LAYOUT>(buf, kWarpBatch, shift, lane, d, (float)(c.x * N + x), (float)(c.y * N + y),
+                       (float)(c.z * N + z), first + (uint32_t)lane, tab);
+  }
+  if (lane_flush) {
+    __syncwarp();
+    flush_warp_lanes<LAYOUT>(buf, shift, nw, g, out0, out1);
+  } else {
+    fence_proxy_async_smem();
+    __syncwarp();
+    flush_warp<LAYOUT>(buf, shift, nw, g, out0, out1);
+  }
+  __syncwarp();
+  b = nbuf == 2 ? b ^ 1 : 0;
+}
+
+// Faces of the batch that starts at global face g with `left` faces to go: a batch that starts
+// off a line_faces boundary of the output ends on a later one, so that the batches after it
+// cover whole 128-byte lines.
+template <int LAYOUT>
+__device__ __forceinline__ int batch_faces(unsigned long long g, int left) {
+  return min(kWarpBatch - (int)(g & (unsigned long long)(line_faces<LAYOUT>() - 1u)), left);
+}
+// The faces of a batch of cnt faces at g that fit an output of cap faces.
+__device__ __forceinline__ int faces_in(unsigned long long g, int cnt, unsigned long long cap) {
+  return g >= cap ? 0 : (g + (unsigned long long)cnt > cap ? (int)(cap - g) : cnt);
+}
+
 // Sends the nwf faces of a warp's face list (chunk-local indices first, first + 1, ...) to
-// global faces g0 + first + ...: 32 at a time staged in one of the warp's nbuf buffers
-// (`bufs`, buffer index b carried across calls) and sent by a TMA bulk copy, or by
-// coalesced lane stores when lane_flush.
+// global faces g0 + first + ..., a batch at a time.
 template <int N, int LAYOUT>
 __device__ __forceinline__ void warp_send_faces(const TablesDev* tab, const uint32_t* list, int nwf,
                                                 uint32_t first, vox_chunk_coord c,
                                                 unsigned long long g0, unsigned long long cap,
                                                 void* out0, void* out1, unsigned char* bufs,
                                                 int nbuf, bool lane_flush, int& b) {
-  constexpr int kBuf = warp_buf_bytes<LAYOUT>();
-  const int ox = c.x * N, oy = c.y * N, oz = c.z * N;
   const int lane = threadIdx.x & 31;
   for (int r0 = 0, cnt = 0; r0 < nwf; r0 += cnt) {
     const unsigned long long g = g0 + first + (unsigned)r0;
-    // a batch that starts off a line_faces boundary of the output ends on a later one, so
-    // that the batches after it cover whole 128-byte lines
-    cnt = kWarpBatch - (int)(g & (unsigned long long)(line_faces<LAYOUT>() - 1u));
-    if (cnt > nwf - r0) cnt = nwf - r0;
-    int nw = cnt;
-    if (g >= cap) nw = 0;
-    else if (g + (unsigned long long)cnt > cap) nw = (int)(cap - g);
+    cnt = batch_faces<LAYOUT>(g, nwf - r0);
+    const int nw = faces_in(g, cnt, cap);
     if (nw == 0) continue;
-    unsigned char* buf = bufs + b * kBuf;
-    // the copy issued nbuf batches ago read this buffer; wait until it is done reading
-    if (lane == 0) {
-      if (nbuf == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-      else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-    }
-    __syncwarp();
-    const int shift = stage_shift<LAYOUT>(g);
-    if (lane < nw) {
-      const uint32_t q = list[r0 + lane];
-      const int x = q & 127, y = (q >> 7) & 127, z = (q >> 14) & 127, d = q >> 21;
-      stage_face<LAYOUT>(buf, kWarpBatch, shift, lane, d, (float)(ox + x), (float)(oy + y),
-                         (float)(oz + z), first + (uint32_t)(r0 + lane), tab);
-    }
-    if (lane_flush) {
-      __syncwarp();
-      flush_warp_lanes<LAYOUT>(buf, shift, nw, g, out0, out1);
-    } else {
-      fence_proxy_async_smem();
-      __syncwarp();
-      flush_warp<LAYOUT>(buf, shift, nw, g, out0, out1);
-    }
-    __syncwarp();
-    b = nbuf == 2 ? b ^ 1 : 0;
+    warp_send_batch<N, LAYOUT>(tab, lane < nw ? list[r0 + lane] : 0u, nw, first + (uint32_t)r0, c, g,
+                               out0, out1, bufs, nbuf, lane_flush, b);
   }
 }
 
-// Emission of elements [lo, hi): warp w takes the contiguous run [lo + w*per, ...) of
-// whole groups of 32 elements, so consecutive groups' faces are adjacent in the output.
+// Emission of elements [lo, hi): part w of `parts` (a warp each) takes the contiguous run
+// [lo + w*per, ...) of whole groups of 32 elements, so consecutive groups' faces are adjacent
+// in the output.
 // Faces accumulate in the warp's list and leave once there are at least 32, up to the last
 // line_faces boundary of the output (g0: the output index of chunk-local face 0); fewer
 // than line_faces are carried to the next group, and the rest leave at the end. Batches
 // that start and end on those boundaries write whole 128-byte lines, which matters most
 // for outputs in host memory, where a partial line costs a slower write.
-template <int N, int LAYOUT, typename Send>
-__device__ __forceinline__ void emit_runs(ChunkSmem<N, LAYOUT>& s, int lo, int hi,
-                                          unsigned long long g0, Send send) {
+template <int N, int LAYOUT, typename Smem, typename Send>
+__device__ __forceinline__ void emit_runs(const Smem& s, int lo, int hi, int part,
+                                          int parts, unsigned long long g0, Send send) {
   constexpr unsigned kLine = line_faces<LAYOUT>();
   const unsigned phase = (unsigned)(g0 & (unsigned long long)(kLine - 1u));
   const bool use_list = s.misc[1] >= 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* list = s.lists + warp * kWarpFaces;
   const int groups = (hi - lo + 31) >> 5;
-  const int gper = (groups + nwarps - 1) / nwarps;
-  const int wlo = lo + warp * gper * 32;
+  const int gper = (groups + parts - 1) / parts;
+  const int wlo = lo + part * gper * 32;
   const int whi = min(hi, wlo + gper * 32);
   int have = 0;             // faces waiting in list[0, have)
   uint32_t first_have = 0;  // chunk-local index of list[0]
   for (int base = wlo; base < whi; base += 32) {
     uint32_t first;
-    const int nwf = warp_faces<N, LAYOUT>(s, use_list, whi, base, list + have, first);
+    const int nwf = warp_faces<N>(s, use_list, whi, base, list + have, first);
     if (have == 0) first_have = first;
     have += nwf;
     const int full = have >= 32 ? have - (int)((phase + first_have + (unsigned)have) & (kLine - 1u)) : 0;
@@ -1836,14 +1906,15 @@ __device__ __forceinline__ void emit_runs(ChunkSmem<N, LAYOUT>& s, int lo, int h
 // so the warp need not wait for its last copies here (with two buffers it still does: the
 // next call starts again at buffer 0, which the last copy may still be reading).
 template <int N, int LAYOUT>
-__device__ void emit_chunk(ChunkSmem<N, LAYOUT>& s, vox_chunk_coord c, unsigned long long g0,
+__device__ void emit_chunk(const ChunkSmem<N, LAYOUT>& s, vox_chunk_coord c, unsigned long long g0,
                            unsigned long long cap, void* out0, void* out1, int nbuf,
-                           bool lane_flush, int lo, int hi, bool wait_read = true) {
+                           bool lane_flush, int lo, int hi, int part, int parts,
+                           bool wait_read = true) {
   constexpr int kBuf = warp_buf_bytes<LAYOUT>();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned char* bufs = s.stage + (size_t)warp * nbuf * kBuf;
   int b = 0;
-  emit_runs<N, LAYOUT>(s, lo, hi, g0, [&](const uint32_t* list, int nf, uint32_t first) {
+  emit_runs<N, LAYOUT>(s, lo, hi, part, parts, g0, [&](const uint32_t* list, int nf, uint32_t first) {
     warp_send_faces<N, LAYOUT>(s.tab, list, nf, first, c, g0, cap, out0, out1, bufs, nbuf,
                                lane_flush, b);
   });
@@ -1902,7 +1973,7 @@ __device__ __forceinline__ void warp_store_faces(const TablesDev* tab, const uin
   const int ox = c.x * N, oy = c.y * N, oz = c.z * N;
   for (int i = threadIdx.x & 31; i < nwf; i += 32) {
     const uint32_t q = list[i];
-    const int x = q & 127, y = (q >> 7) & 127, z = (q >> 14) & 127, d = q >> 21;
+    const int x = q & 255, y = (q >> 8) & 255, z = (q >> 16) & 255, d = q >> 24;
     const uint32_t l = first + (uint32_t)i;
     const unsigned long long gg = g0 + l;
     if (gg < cap)
@@ -1915,12 +1986,152 @@ __device__ __forceinline__ void warp_store_faces(const TablesDev* tab, const uin
 // Direct variant of emit_chunk: the same runs and compaction, then every lane writes one
 // face record straight to global memory (32 consecutive faces per warp step).
 template <int N, int LAYOUT>
-__device__ void emit_chunk_direct(ChunkSmem<N, LAYOUT>& s, vox_chunk_coord c,
+__device__ void emit_chunk_direct(const ChunkSmem<N, LAYOUT>& s, vox_chunk_coord c,
                                   unsigned long long g0, unsigned long long cap, void* out0,
-                                  void* out1, int lo, int hi) {
-  emit_runs<N, LAYOUT>(s, lo, hi, g0, [&](const uint32_t* list, int nf, uint32_t first) {
+                                  void* out1, int lo, int hi, int part, int parts) {
+  emit_runs<N, LAYOUT>(s, lo, hi, part, parts, g0, [&](const uint32_t* list, int nf, uint32_t first) {
     warp_store_faces<N, LAYOUT>(s.tab, list, nf, first, c, g0, cap, out0, out1);
   });
+}
+
+// A chunk's face list (overlap schedule): one packed face (pack_face) per face in emission
+// order, in the chunk's spill slot, written by the generation item from the face voxels and
+// read by the emission item, which then needs no chunk state in shared memory, no compaction
+// and no barrier beyond the offset's. It takes 4 bytes a face next to the 68 or 120 it
+// describes. Chunks with more faces than the slot holds, kMiscOff / 4 (7 N^2 to 10 N^2 up to
+// 32^3, 3.7 N^2 at 64^3; terrain has 2 N^2 to 4 N^2, random voxels 100 N^2), spill their
+// occupancy and row lists instead and are compacted at emission.
+// Position of set bit n (from 0) of m, which has more than n.
+template <int N, typename RowT>
+__device__ __forceinline__ int nth_bit(RowT m, int n) {
+  int pos = 0;
+#pragma unroll
+  for (int w = N / 2; w > 0; w >>= 1) {
+    const int c = popc_row((RowT)(m & (((RowT)1 << w) - (RowT)1)));
+    if (n >= c) {
+      n -= c;
+      m >>= w;
+      pos += w;
+    }
+  }
+  return pos;
+}
+
+// 64^3 chunks have no voxel list: a warp takes 32 rows at a time, dealt out over the warps so
+// that neighbouring rows (which have faces together) go to different ones, counts the face
+// voxels of each, and then every lane finds its own voxel among them by search. (Going
+// through all 64 voxels of every row with faces left nine lanes in ten idle: 30 terrain chunks
+// of 64^3 took 380 us a batch, 127 us this way. Where the voxels are listed the search costs
+// more than it saves: at 32^3 a batch of 777 cave chunks took 57 us instead of 45.)
+template <int N, int LAYOUT>
+__device__ __forceinline__ void write_face_rows(const ChunkSmem<N, LAYOUT>& s, uint32_t* dst) {
+  using RowT = typename Shape<N>::RowT;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  for (int r0 = 0; r0 < N * N; r0 += 32 * nwarps) {
+    RowT m[6];
+    const int mine = r0 + lane * nwarps + warp;
+    const bool faces = s.rows[mine + 1] != s.rows[mine];
+    if (__all_sync(0xffffffffu, !faces)) continue;
+    int cnt = 0;
+    if (faces) {
+      row_masks<N, LAYOUT>(s, mine / N, mine % N, m);
+      cnt = popc_row((RowT)(m[0] | m[1] | m[2] | m[3] | m[4] | m[5]));
+    }
+    int incl = cnt;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += v;
+    }
+    const int voxels = __shfl_sync(0xffffffffu, incl, 31);
+    for (int base = 0; base < voxels; base += 32) {
+      const int k = base + lane;
+      int own = 0;  // the lane whose row holds voxel k: the first with incl > k
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, incl, own + step - 1) <= k) own += step;
+      const int before = __shfl_sync(0xffffffffu, incl - cnt, own);
+      if (k < voxels) {
+        const int r = r0 + own * nwarps + warp, y = r / N, z = r % N;
+        row_masks<N, LAYOUT>(s, y, z, m);
+        const int x = nth_bit<N>((RowT)(m[0] | m[1] | m[2] | m[3] | m[4] | m[5]), k - before);
+        const RowT below = ((RowT)1 << x) - (RowT)1;
+        uint32_t* out = dst + s.rows[r];
+        unsigned bits = 0;
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+          out += popc_row((RowT)(m[d] & below));
+          bits |= (unsigned)((m[d] >> x) & (RowT)1) << d;
+        }
+        const uint32_t code = pack_face(x, y, z, 0);
+        while (bits) {
+          const int d = __ffs(bits) - 1;
+          bits &= bits - 1u;
+          *out++ = code | ((uint32_t)d << 24);
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+template <int N, int LAYOUT>
+__device__ __forceinline__ void write_face_list(const ChunkSmem<N, LAYOUT>& s, uint32_t* dst) {
+  if constexpr (Shape<N>::VCap == 0) {
+    write_face_rows<N, LAYOUT>(s, dst);
+  } else {
+    const bool use_list = s.misc[1] >= 0;
+    const int elems = emit_elems(s);
+    for (int base = (int)(threadIdx.x & ~31u); base < elems; base += blockDim.x) {
+      uint32_t first;
+      warp_faces<N, true>(s, use_list, elems, base, dst, first);
+    }
+  }
+}
+
+// Emission of part `part` of `parts` (a warp each) of a chunk from its face list (`total` faces,
+// the chunk's first at global face g0): the output lines that the chunk touches are cut
+// evenly over the parts, so every batch but the chunk's first and last covers whole lines.
+template <int N, int LAYOUT>
+__device__ __forceinline__ void emit_list(const ChunkSmem<N, LAYOUT>& s, const uint32_t* codes,
+                                          uint32_t total, unsigned part, unsigned parts,
+                                          vox_chunk_coord c, unsigned long long g0,
+                                          unsigned long long cap, void* out0, void* out1, int nbuf,
+                                          bool lane_flush) {
+  constexpr unsigned kLine = line_faces<LAYOUT>();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned phase = (unsigned)(g0 & (unsigned long long)(kLine - 1u));
+  const unsigned lines = (phase + total + kLine - 1u) / kLine;
+  const unsigned la = lines * part / parts, lb = lines * (part + 1u) / parts;
+  if (la == lb) return;
+  const int lo = la == 0u ? 0 : (int)(la * kLine - phase);
+  const int hi = (int)min(total, lb * kLine - phase);
+  unsigned char* bufs = s.stage + (size_t)warp * nbuf * warp_buf_bytes<LAYOUT>();
+  int b = 0;
+  int cnt = batch_faces<LAYOUT>(g0 + (unsigned)lo, hi - lo);
+  uint32_t q = lane < cnt ? __ldcg(codes + lo + lane) : 0u;
+  for (int r = lo; r < hi;) {
+    const unsigned long long g = g0 + (unsigned)r;
+    const int r2 = r + cnt;
+    const int cnt2 = r2 < hi ? batch_faces<LAYOUT>(g0 + (unsigned)r2, hi - r2) : 0;
+    const uint32_t q2 = lane < cnt2 ? __ldcg(codes + r2 + lane) : 0u;  // the next batch's faces
+    const int nw = faces_in(g, cnt, cap);
+    if (nw == 0) break;
+    if (nbuf > 0) {
+      warp_send_batch<N, LAYOUT>(s.tab, q, nw, (uint32_t)r, c, g, out0, out1, bufs, nbuf, lane_flush, b);
+    } else if (lane < nw) {
+      const int x = q & 255, y = (q >> 8) & 255, z = (q >> 16) & 255, d = q >> 24;
+      store_face<LAYOUT>(out0, out1, g + (unsigned)lane, d, (float)(c.x * N + x), (float)(c.y * N + y),
+                         (float)(c.z * N + z), (uint32_t)(r + lane), s.tab);
+    }
+    r = r2;
+    cnt = cnt2;
+    q = q2;
+  }
+  if (nbuf > 1) {  // the next item starts at buffer 0 again (one buffer: its first send waits)
+    if (lane == 0) bulk_wait_read_all();
+    __syncwarp();
+  }
 }
 
 // ------------------------------------------------------------------------------------
@@ -1949,7 +2160,7 @@ __host__ __device__ constexpr int fused_min_ctas() {
 // meshing of resident occupancy (GM == GM_OCC). One chunk per CTA iteration; T threads.
 // Occupancy and halo rows of chunk i in shared memory: loaded from the slot pool
 // (GM_OCC) or generated from the noise field.
-template <int N, int GM, int LAYOUT, int T>
+template <int N, int GM, int LAYOUT, int T, bool kHashed = false>
 __device__ __forceinline__ void prepare_chunk(ChunkSmem<N, LAYOUT>& s, const MeshArgs& a, int i,
                                               vox_chunk_coord c) {
   if (GM == GM_OCC) {
@@ -1976,7 +2187,7 @@ __device__ __forceinline__ void prepare_chunk(ChunkSmem<N, LAYOUT>& s, const Mes
     unsigned m = a.nbr_mask ? a.nbr_mask[i] : 0u;
     if (GM == GM_BERNOULLI) m = 0u;
     if (!a.full6) m &= 0xFu;
-    gen_chunk<N, GM, LAYOUT, T>(s, a.gen, c, a.index_base + i, m, true);
+    gen_chunk<N, GM, LAYOUT, T, kHashed>(s, a.gen, c, a.index_base + i, m, true);
   }
 }
 
@@ -2032,8 +2243,9 @@ k_mesh_batch(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
     __syncthreads();
     if (a.stage_faces > 0)
       emit_chunk<N, LAYOUT>(s, c, s_base, a.cap, a.out0, a.out1, a.stage_faces / kWarpBatch,
-                            a.lane_flush != 0, 0, emit_elems(s));
-    else emit_chunk_direct<N, LAYOUT>(s, c, s_base, a.cap, a.out0, a.out1, 0, emit_elems(s));
+                            a.lane_flush != 0, 0, emit_elems(s), threadIdx.x >> 5, T / 32);
+    else emit_chunk_direct<N, LAYOUT>(s, c, s_base, a.cap, a.out0, a.out1, 0, emit_elems(s),
+                                        threadIdx.x >> 5, T / 32);
     if (threadIdx.x == 0) s_item = next_item;
     __syncthreads();
     i = s_item;
@@ -2273,8 +2485,8 @@ k_mesh_batch_phased(const __grid_constant__ MeshArgs a, const __grid_constant__ 
       const vox_chunk_coord c = a.coords[i];
       if (a.stage_faces > 0)
         emit_chunk<N, LAYOUT>(s, c, s_base, a.cap, a.out0, a.out1, a.stage_faces / kWarpBatch,
-                              a.lane_flush != 0, lo, hi, false);
-      else emit_chunk_direct<N, LAYOUT>(s, c, s_base, a.cap, a.out0, a.out1, lo, hi);
+                              a.lane_flush != 0, lo, hi, t >> 5, T / 32, false);
+      else emit_chunk_direct<N, LAYOUT>(s, c, s_base, a.cap, a.out0, a.out1, lo, hi, t >> 5, T / 32);
     }
     if (t == 0) s_item = next_item;
     __syncthreads();
@@ -2306,6 +2518,8 @@ k_mesh_batch_overlap(const __grid_constant__ MeshArgs a, const __grid_constant__
   constexpr int kVlOff = kNzOff + P::kNz;
   constexpr int kMiscOff = kVlOff + P::kVList;
   static_assert(P::kSpill == kMiscOff + P::kMisc, "spill layout");
+  constexpr uint32_t kListCap = kMiscOff / 4;  // faces of a face list (see write_face_list)
+  constexpr int kListed = -2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ChunkSmem<N, LAYOUT> s;
   s.carve(smem_raw);
@@ -2361,20 +2575,26 @@ k_mesh_batch_overlap(const __grid_constant__ MeshArgs a, const __grid_constant__
       prepare_chunk<N, GM, LAYOUT, T>(s, a, i, a.coords[i]);
       const uint32_t total = count_and_scan<N, LAYOUT, T>(s);
       unsigned char* dst = spill + (unsigned long long)i * P::kSpill;
-      // an empty chunk (no row with faces) spills only its counts: its emission item
-      // reloads nothing
-      if (s.misc[0] > 0)
+      // the chunk's face list, or its state when the list does not fit the slot; an empty
+      // chunk (no row with faces) spills only its counts
+      const bool listed = total <= kListCap;
+      if (listed) {
+        write_face_list<N, LAYOUT>(s, reinterpret_cast<uint32_t*>(dst));
+      } else {
         for (int q = t; q < kFixed16; q += T) __stcg(reinterpret_cast<uint4*>(dst) + q, fixed16[q]);
-      const int nzw = (s.misc[0] + 1) >> 1;
-      const int vlw = s.misc[1] > 0 ? (s.misc[1] + 1) >> 1 : 0;
-      for (int q = t; q < nzw; q += T)
-        __stcg(reinterpret_cast<uint32_t*>(dst + kNzOff) + q, reinterpret_cast<const uint32_t*>(s.nz)[q]);
-      for (int q = t; q < vlw; q += T)
-        __stcg(reinterpret_cast<uint32_t*>(dst + kVlOff) + q,
-               reinterpret_cast<const uint32_t*>(s.vlist)[q]);
+        const int nzw = (s.misc[0] + 1) >> 1;
+        const int vlw = s.misc[1] > 0 ? (s.misc[1] + 1) >> 1 : 0;
+        for (int q = t; q < nzw; q += T)
+          __stcg(reinterpret_cast<uint32_t*>(dst + kNzOff) + q, reinterpret_cast<const uint32_t*>(s.nz)[q]);
+        for (int q = t; q < vlw; q += T)
+          __stcg(reinterpret_cast<uint32_t*>(dst + kVlOff) + q,
+                 reinterpret_cast<const uint32_t*>(s.vlist)[q]);
+      }
       __syncthreads();  // every store of the slot precedes the publication below
       if (t == 0) {
-        __stcg(reinterpret_cast<int2*>(dst + kMiscOff), make_int2(s.misc[0], s.misc[1]));
+        // {faces, kListed} or {rows with faces, face voxels or -1}
+        __stcg(reinterpret_cast<int2*>(dst + kMiscOff),
+               listed ? make_int2((int)total, kListed) : make_int2(s.misc[0], s.misc[1]));
         __threadfence();
         st_relaxed_u64(&a.state[i], pack_state(epoch, i == 0 ? kFlagIncl : kFlagAgg, total));
       }
@@ -2400,19 +2620,21 @@ k_mesh_batch_overlap(const __grid_constant__ MeshArgs a, const __grid_constant__
       ok = __all_sync(0xffffffffu, ok);  // warp-uniform (warp 0's look-back needs every lane)
       if (!ok && (t & 31) == 0) atomicOr(&a.ctl->err, ERR_TIMEOUT);
       // Warp 0 takes the chunk's offset by look-back over the published totals while the
-      // other warps reload the chunk's state (a one-warp CTA does both, in turn).
+      // other warps reload the chunk's state if it has no face list (a one-warp CTA does
+      // both, in turn).
       constexpr int TR = T > 32 ? T - 32 : 32;  // reloading threads
       const int tr = T > 32 ? t - 32 : t;
+      int2 m = make_int2(0, kListed);
+      if (ok) m = __ldcg(reinterpret_cast<const int2*>(src + kMiscOff));
+      const bool listed = m.y == kListed;
       if (t < 32 && ok) {
-        // the chunk's face total (an empty chunk spilled only its counts: total 0)
-        const int rows_with_faces = __ldcg(reinterpret_cast<const int*>(src + kMiscOff));
+        // the chunk's face total
         const unsigned long long total =
-            rows_with_faces > 0
-                ? __ldcg(reinterpret_cast<const uint32_t*>(src + P::kOcc + P::kHalo) + Shape<N>::R)
-                : 0ull;
+            listed ? (unsigned long long)m.x
+                   : __ldcg(reinterpret_cast<const uint32_t*>(src + P::kOcc + P::kHalo) + Shape<N>::R);
+        w = __shfl_sync(0xffffffffu, w, 0);
         // An inclusive state (chunk 0, or a segment of a chunk whose offset another item
         // has already found) gives the offset at once.
-        w = __shfl_sync(0xffffffffu, w, 0);
         const unsigned long long excl =
             base0 + (((w >> 38) & 3ull) == kFlagIncl
                          ? (w & ((1ull << 38) - 1)) - total
@@ -2428,38 +2650,45 @@ k_mesh_batch_overlap(const __grid_constant__ MeshArgs a, const __grid_constant__
           }
         }
       }
-      if (ok && tr >= 0) {
-        const int2 m = __ldcg(reinterpret_cast<const int2*>(src + kMiscOff));
+      if (ok && !listed && tr >= 0) {
         if (tr == 0) {
           s.misc[0] = m.x;
           s.misc[1] = m.y;
         }
-        if (m.x > 0) {  // rows with faces: an empty chunk needs no state
-          for (int q = tr; q < kFixed16; q += TR) fixed16[q] = __ldcg(reinterpret_cast<const uint4*>(src) + q);
-          const bool use_list = m.y >= 0;
-          const int elems = use_list ? m.y : m.x * N;
-          const int per = ((elems + split - 1) / split + 31) & ~31;
-          const int lo = min(elems, seg * per), hi = min(elems, lo + per);
-          if (lo < hi) {
-            const int e0 = use_list ? lo : lo / N, e1 = use_list ? hi : (hi - 1) / N + 1;
-            const uint32_t* lsrc = reinterpret_cast<const uint32_t*>(src + (use_list ? kVlOff : kNzOff));
-            uint32_t* ldst = reinterpret_cast<uint32_t*>(use_list ? s.vlist : s.nz);
-            for (int q = (e0 >> 1) + tr; q < (e1 + 1) >> 1; q += TR) ldst[q] = __ldcg(lsrc + q);
-          }
+        for (int q = tr; q < kFixed16; q += TR) fixed16[q] = __ldcg(reinterpret_cast<const uint4*>(src) + q);
+        const bool use_list = m.y >= 0;
+        const int elems = use_list ? m.y : m.x * N;
+        const int per = ((elems + split - 1) / split + 31) & ~31;
+        const int lo = min(elems, seg * per), hi = min(elems, lo + per);
+        if (lo < hi) {
+          const int e0 = use_list ? lo : lo / N, e1 = use_list ? hi : (hi - 1) / N + 1;
+          const uint32_t* lsrc = reinterpret_cast<const uint32_t*>(src + (use_list ? kVlOff : kNzOff));
+          uint32_t* ldst = reinterpret_cast<uint32_t*>(use_list ? s.vlist : s.nz);
+          for (int q = (e0 >> 1) + tr; q < (e1 + 1) >> 1; q += TR) ldst[q] = __ldcg(lsrc + q);
         }
       }
       if (!__syncthreads_and(ok)) break;  // never published (error reported)
-      const int elems = emit_elems(s);
-      const int per = ((elems + split - 1) / split + 31) & ~31;
-      const int lo = min(elems, seg * per), hi = min(elems, lo + per);
-      if (lo < hi) {
-        const vox_chunk_coord c = a.coords[c_i];
-        if (a.stage_faces > 0) {
-          emit_chunk<N, LAYOUT>(s, c, s_base, a.cap, a.out0, a.out1, a.stage_faces / kWarpBatch,
-                                a.lane_flush != 0, lo, hi, false);
+      const vox_chunk_coord c = a.coords[c_i];
+      if (listed) {
+        if (m.x > 0) {
+          emit_list<N, LAYOUT>(s, reinterpret_cast<const uint32_t*>(src), (uint32_t)m.x,
+                               (unsigned)(seg * (T / 32) + (t >> 5)), (unsigned)(split * (T / 32)), c,
+                               s_base, a.cap, a.out0, a.out1, a.stage_faces / kWarpBatch,
+                               a.lane_flush != 0);
           stage_busy = true;
-        } else {
-          emit_chunk_direct<N, LAYOUT>(s, c, s_base, a.cap, a.out0, a.out1, lo, hi);
+        }
+      } else {
+        const int elems = emit_elems(s);
+        const int per = ((elems + split - 1) / split + 31) & ~31;
+        const int lo = min(elems, seg * per), hi = min(elems, lo + per);
+        if (lo < hi) {
+          if (a.stage_faces > 0) {
+            emit_chunk<N, LAYOUT>(s, c, s_base, a.cap, a.out0, a.out1, a.stage_faces / kWarpBatch,
+                                  a.lane_flush != 0, lo, hi, t >> 5, T / 32, false);
+            stage_busy = true;
+          } else {
+            emit_chunk_direct<N, LAYOUT>(s, c, s_base, a.cap, a.out0, a.out1, lo, hi, t >> 5, T / 32);
+          }
         }
       }
     }
@@ -2490,8 +2719,9 @@ k_mesh_single(MeshArgs a) {
   }
   if (a.stage_faces > 0)
     emit_chunk<N, LAYOUT>(s, a.coord_single, 0ull, a.cap, a.out0, a.out1, a.stage_faces / kWarpBatch,
-                          a.lane_flush != 0, 0, emit_elems(s));
-  else emit_chunk_direct<N, LAYOUT>(s, a.coord_single, 0ull, a.cap, a.out0, a.out1, 0, emit_elems(s));
+                          a.lane_flush != 0, 0, emit_elems(s), threadIdx.x >> 5, T / 32);
+  else emit_chunk_direct<N, LAYOUT>(s, a.coord_single, 0ull, a.cap, a.out0, a.out1, 0, emit_elems(s),
+                                        threadIdx.x >> 5, T / 32);
   if ((threadIdx.x & 31) == 0) bulk_wait_all();
 }
 
@@ -2525,8 +2755,10 @@ k_generate(MeshArgs a, uint32_t* occ_out) {
     }
   }
   load_tables<N, VOX_LAYOUT_VERTEX>(s, a.tables);
+  constexpr bool kHashed = GM == GM_HEIGHT && N <= 32;
+  if (kHashed) load_grad2<T>(s, reinterpret_cast<float2*>(s.stage), a.grad2);
   __syncthreads();
-  gen_chunk<N, GM, VOX_LAYOUT_VERTEX, T>(s, a.gen, a.coords[i], a.index_base + i, 0u, false);
+  gen_chunk<N, GM, VOX_LAYOUT_VERTEX, T, kHashed>(s, a.gen, a.coords[i], a.index_base + i, 0u, false);
   const uint32_t* src = reinterpret_cast<const uint32_t*>(s.occ);
   uint32_t* dst = occ_out + (size_t)slot * words;
   for (int q = threadIdx.x; q < words; q += blockDim.x) dst[q] = src[q];
@@ -2567,7 +2799,7 @@ k_generate_planes(MeshArgs a, const uint8_t* __restrict__ dirs, uint32_t* occ_ou
       const int z = d <= 1 ? q : (d <= 3 ? fix : p);
       bool solid;
       if constexpr (GM == GM_HEIGHT)
-        solid = y < column_k<N, VOX_LAYOUT_VERTEX>(s, a.gen, ox, oy, oz, x, z);
+        solid = y < column_k<N>(s, a.gen, ox, oy, oz, x, z);
       else
         solid = gen_solid<N, GM, VOX_LAYOUT_VERTEX>(s, a.gen, x, y, z, ox, oy, oz, 0ull);
       if (solid) atomicOr(&occw[(y * N + z) * W + (x >> 5)], 1u << (x & 31));

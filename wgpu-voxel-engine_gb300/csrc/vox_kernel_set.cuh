@@ -3,6 +3,7 @@
 
 #include "vox_device.cuh"
 #include "vox_kernels.h"
+#include "vox_lists.cuh"
 
 namespace vox {
 
@@ -23,6 +24,15 @@ static void fill_batch(KernelSet& k) {
   k.overlap[GM][L][1] = (const void*)k_mesh_batch_overlap<N, GM, L, Shape<N>::T1>;
 }
 
+template <int N, int GM>
+static void fill_lists(KernelSet& k) {
+  k.list[GM][0] = (const void*)k_list_chunks<N, GM, 0>;
+  // (two CTA sizes only where they differ)
+  k.list[GM][1] = list_threads<N>(1) == list_threads<N>(0) ? k.list[GM][0]
+                                                           : (const void*)k_list_chunks<N, GM, (N > 16)>;
+  k.list_smem[GM] = ListSmem<N, GM>::kBytes;
+}
+
 template <int N>
 static KernelSet make_kernel_set() {
   KernelSet k{};
@@ -41,6 +51,15 @@ static KernelSet make_kernel_set() {
   k.single[0][1] = (const void*)k_mesh_single<N, VOX_LAYOUT_VERTEX, Shape<N>::T1>;
   k.single[1][0] = (const void*)k_mesh_single<N, VOX_LAYOUT_INSTANCED, Shape<N>::T0>;
   k.single[1][1] = (const void*)k_mesh_single<N, VOX_LAYOUT_INSTANCED, Shape<N>::T1>;
+  fill_lists<N, GM_OCC>(k);
+  fill_lists<N, GM_HEIGHT>(k);
+  fill_lists<N, GM_DENSITY>(k);
+  k.emit[VOX_LAYOUT_VERTEX] = (const void*)k_emit_lists<N, VOX_LAYOUT_VERTEX>;
+  k.emit[VOX_LAYOUT_INSTANCED] = (const void*)k_emit_lists<N, VOX_LAYOUT_INSTANCED>;
+  k.emit_threads = kEmitThreads;
+  k.list_threads[0] = list_threads<N>(0);
+  k.list_threads[1] = list_threads<N>(1);
+  k.list_slot_bytes = ListSlot<N>::kBytes;
   k.gen_threads = Shape<N>::T1;
   k.spill_bytes = SmemPlan<N, VOX_LAYOUT_VERTEX>::kSpill;
   k.generate[0] = nullptr;

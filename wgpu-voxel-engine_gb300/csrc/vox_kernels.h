@@ -16,6 +16,12 @@ struct KernelSet {
   const void* single[2][2];     // k_mesh_single<N, layout, threads[t]>
   const void* generate[4];      // k_generate<N, gen mode, gen_threads> (index 0 unused)
   const void* generate_planes[4]; // k_generate_planes<N, gen mode, gen_threads> (height, density)
+  // the list launches (vox_lists.cuh); none for Bernoulli chunks, which have too many faces
+  const void* list[4][2];       // k_list_chunks<N, gen mode, list_threads[t]>
+  int list_threads[2], list_smem[4];
+  const void* emit[2];          // k_emit_lists<N, layout>
+  int emit_threads;
+  int list_slot_bytes;          // scratch of one chunk
   int gen_threads;
   int spill_bytes;              // chunk state of one chunk (phased scratch)
   // dynamic shared memory of a launch (layout, CTA size, staging window in faces)

@@ -1,0 +1,461 @@
+// vox_lists.cuh — the two launches of a batch under the overlap schedule with outputs in device
+// memory: k_list_chunks generates (or loads) and counts one chunk per CTA and writes its faces
+// as a list of 4-byte codes, k_emit_lists turns the lists into records.
+//
+// One persistent launch for both (k_mesh_batch_overlap) gives every CTA the registers and the
+// shared memory of the hungrier half: 4 CTAs of 256 threads an SM for 16^3 terrain, whose chunks
+// then need two waves and whose emission waits behind CTA barriers (a chunk in 6.4 us, twice, then
+// as long for its emission). Split, generation runs at the occupancy of its own needs (8 CTAs,
+// all 1024 chunks at once, the last done after 14 us), and emission has no CTA barriers: a
+// warp takes a part of a chunk, reads its codes and writes whole 128-byte lines. The second
+// launch is a programmatic dependent of the first (its CTAs start as soon as the last
+// generation CTA has started, and wait for chunks, not for the kernel), so splitting costs no
+// launch gap.
+// Measured, us a batch, one launch -> two: 1024 terrain chunks of 16^3 39.6 -> 33.9, 64 start
+// chunks of 32^3 as instances 41.6 -> 21.7, 777 cave chunks of 32^3 from occupancy 62 -> 42,
+// 4096 cave chunks generated 285 -> 279. What bounds them: generation by its instructions
+// (57 % of issue at 16^3), emission by the offsets' way (the slowest chunk of a group, its scan,
+// the poll: about 4 us) and then the writes (61 MB in 11 us into L2, 4.4 TB/s into HBM).
+#pragma once
+
+#include "vox_device.cuh"
+
+namespace vox {
+
+// Slot of a chunk in the scratch: its face list, or (more faces than the list holds) the spilled
+// chunk state of SmemPlan. The list holds 7 N^2 to 10 N^2 faces up to 32^3 (the size of
+// the chunk state) and 8 N^2 at 64^3; terrain has 2 N^2 to 4 N^2, random voxels 100 N^2.
+template <int N>
+struct ListSlot {
+  using P = SmemPlan<N, VOX_LAYOUT_VERTEX>;
+  static constexpr int kNzOff = P::kOcc + P::kHalo + P::kRows;
+  static constexpr int kVlOff = kNzOff + P::kNz;
+  static constexpr int kMiscOff = kVlOff + P::kVList;
+  static constexpr int kBytes = N == 64 ? 8 * N * N * 4 : P::kSpill;
+  static constexpr uint32_t kCap = kBytes / 4;
+  static_assert(kBytes >= P::kSpill, "the slot holds a spilled chunk state");
+};
+
+// CTA sizes of k_list_chunks: kBig = 0 for many chunks; kBig = 1, up to one thread a row, for
+// batches of no more chunks than SMs, where a chunk's latency is the batch's.
+template <int N>
+__host__ __device__ constexpr int list_threads(int big) {
+  return N == 8 ? 64 : (N == 16 ? 256 : (N == 32 ? (big ? 1024 : 256) : (big ? 1024 : 512)));
+}
+
+// Dynamic shared memory of k_list_chunks: tables, occupancy, halo and counts, then the row
+// offsets, row and voxel lists and the count's warp totals, which take the place of the
+// generator's scratch once the occupancy is there.
+template <int N, int GM>
+struct ListSmem {
+  using P = SmemPlan<N, VOX_LAYOUT_VERTEX>;
+  static constexpr int kRowsOff = P::kTables + P::kOcc + P::kHalo + P::kMisc;
+  static constexpr int kLists = P::kRows + P::kNz + P::kVList;
+  static constexpr int kScratch = GM == GM_DENSITY  ? dens_scratch_bytes<N>()
+                                  : GM == GM_HEIGHT ? (N > 32 ? P::kHeight : kGrad2 * 8)
+                                                    : 0;
+  static constexpr int kBytes = kRowsOff + (kScratch > kLists + 256 ? kScratch : kLists + 256);
+};
+
+// Resident CTAs per SM that k_list_chunks is compiled for (its register budget): 64 registers
+// for the density evaluation and for 64^3 chunks, 32 otherwise.
+template <int N, int GM, int kBig>
+__host__ __device__ constexpr int list_min_ctas() {
+  constexpr int kCtas = 65536 / (list_threads<N>(kBig) * (GM == GM_DENSITY || N == 64 ? 64 : 32));
+  return kCtas < 32 ? kCtas : 32;
+}
+
+template <int N, int GM, int kBig>
+__global__ void __launch_bounds__(list_threads<N>(kBig), list_min_ctas<N, GM, kBig>())
+k_list_chunks(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesDev tab) {
+  using P = SmemPlan<N, VOX_LAYOUT_VERTEX>;
+  using S = ListSlot<N>;
+  constexpr int T = list_threads<N>(kBig);
+  // the dependent launch may start once every CTA is past this point
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  using M = ListSmem<N, GM>;
+  ChunkSmem<N, VOX_LAYOUT_VERTEX> s;
+  s.carve(smem_raw, 0);
+  s.misc = reinterpret_cast<int*>(smem_raw + P::kTables + P::kOcc + P::kHalo);
+  unsigned char* const lists = smem_raw + M::kRowsOff;
+  s.rows = reinterpret_cast<uint32_t*>(lists);
+  s.nz = reinterpret_cast<uint16_t*>(lists + P::kRows);
+  s.vlist = reinterpret_cast<uint16_t*>(lists + P::kRows + P::kNz);
+  s.scratch_at(lists);
+  const int i = blockIdx.x, t = threadIdx.x;
+  unsigned epoch = 0;
+  if (t == 0) epoch = ld_relaxed_u32(&a.ctl->epoch);
+  const vox_chunk_coord c = a.coords[i];
+  constexpr bool kHashed = GM == GM_HEIGHT && N <= 32;
+  if (GM != GM_OCC) {
+    load_tables<N, VOX_LAYOUT_VERTEX>(s, &tab);
+    if (kHashed) load_grad2<T>(s, reinterpret_cast<float2*>(lists), a.grad2);
+    __syncthreads();
+  }
+  prepare_chunk<N, GM, VOX_LAYOUT_VERTEX, T, kHashed>(s, a, i, c);
+  s.stage = lists + M::kLists;
+  const uint32_t total = count_and_scan<N, VOX_LAYOUT_VERTEX, T>(s);
+  unsigned char* dst = reinterpret_cast<unsigned char*>(a.scratch) + (unsigned long long)i * S::kBytes;
+  if (total <= S::kCap) {
+    write_face_list<N, VOX_LAYOUT_VERTEX>(s, reinterpret_cast<uint32_t*>(dst));
+  } else {
+    constexpr int kOccHalo = (P::kOcc + P::kHalo) / 16, kRows = P::kRows / 16;
+    for (int q = t; q < kOccHalo + kRows; q += T)  // s.halo follows s.occ
+      __stcg(reinterpret_cast<uint4*>(dst) + q,
+             q < kOccHalo ? reinterpret_cast<const uint4*>(s.occ)[q]
+                          : reinterpret_cast<const uint4*>(s.rows)[q - kOccHalo]);
+    const int nzw = (s.misc[0] + 1) >> 1;
+    const int vlw = s.misc[1] > 0 ? (s.misc[1] + 1) >> 1 : 0;
+    for (int q = t; q < nzw; q += T)
+      __stcg(reinterpret_cast<uint32_t*>(dst + S::kNzOff) + q, reinterpret_cast<const uint32_t*>(s.nz)[q]);
+    for (int q = t; q < vlw; q += T)
+      __stcg(reinterpret_cast<uint32_t*>(dst + S::kVlOff) + q,
+             reinterpret_cast<const uint32_t*>(s.vlist)[q]);
+    if (t == 0) __stcg(reinterpret_cast<int2*>(dst + S::kMiscOff), make_int2(s.misc[0], s.misc[1]));
+  }
+  __syncthreads();  // every store of the slot precedes the publication below
+  if (t == 0) {
+    __threadfence();
+    st_relaxed_u64(&a.state[i], pack_state(epoch, i == 0 ? kFlagIncl : kFlagAgg, total));
+  }
+}
+
+// Offsets. k_list_chunks publishes its chunks' totals as aggregate states. A scan item, one warp
+// per group of kGroup chunks, waits for the group's totals, scans them, takes the group's base by
+// look-back over the group states (behind the n chunk states) and upgrades the chunk states to
+// inclusive prefixes, so that an emission item only waits for two neighbouring words. Letting
+// each emission warp look back itself reads the same few words thousands of times (the
+// 1024-chunk 16^3 terrain in one persistent launch: 42.6 us against 36.0 us).
+constexpr int kGroup = 32;
+static_assert(kGroup == kStateGroup, "the host sizes the states by groups");
+
+__device__ __forceinline__ bool state_valid(unsigned long long w, unsigned tag) {
+  return ((unsigned)(w >> 40) & 0xFFFFFFu) == tag && ((w >> 38) & 3ull) != 0ull;
+}
+
+// Scan item g (one warp). Returns false after a timeout (error bit set).
+static __device__ bool scan_group(const MeshArgs& a, unsigned epoch, int g, unsigned long long base0) {
+  const int lane = threadIdx.x & 31, i = g * kGroup + lane;
+  const unsigned tag = epoch & 0xFFFFFFu;
+  unsigned long long w = 0;
+  for (int spins = 0;;) {
+    if (i < a.n) w = ld_acquire_u64(&a.state[i]);
+    if (__all_sync(0xffffffffu, i >= a.n || state_valid(w, tag))) break;
+    if (++spins > a.spin_limit) {
+      if (lane == 0) atomicOr(&a.ctl->err, ERR_TIMEOUT);
+      return false;
+    }
+    __nanosleep(spins < 8 ? 32 : 128);
+  }
+  const unsigned total = i < a.n ? (unsigned)w : 0u;  // below 2^20; a group's below 2^25
+  unsigned incl = total;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned v = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += v;
+  }
+  const unsigned sum = __shfl_sync(0xffffffffu, incl, 31);
+  const unsigned long long excl = lookback(a.state + a.n, a.ctl, epoch, g, sum, a.spin_limit);
+  __threadfence();  // the chunks' stores, seen by the acquire above, precede the upgrade
+  if (i < a.n) {
+    st_relaxed_u64(&a.state[i], pack_state(epoch, kFlagIncl, excl + incl));
+    a.face_offsets[i] = base0 + excl + incl - total;
+    if (i == a.n - 1) {
+      const unsigned long long end = base0 + excl + incl;
+      a.face_offsets[a.n] = end;
+      if (end > a.cap) atomicOr(&a.ctl->err, ERR_CAPACITY);
+    }
+  }
+  return true;
+}
+
+// Waits for chunk i's offset and total (one warp). Returns false after a timeout.
+static __device__ bool chunk_offset(const MeshArgs& a, unsigned epoch, int i, unsigned long long& excl,
+                                    unsigned& total) {
+  const int lane = threadIdx.x & 31, idx = i - 1 + lane;  // lanes 0 and 1: chunks i - 1 and i
+  const unsigned tag = epoch & 0xFFFFFFu;
+  unsigned long long w = pack_state(epoch, kFlagIncl, 0);
+  for (int spins = 0;;) {
+    if (lane < 2 && idx >= 0) w = ld_acquire_u64(&a.state[idx]);
+    const bool ready = state_valid(w, tag) && ((w >> 38) & 3ull) == kFlagIncl;
+    if (__all_sync(0xffffffffu, ready)) break;
+    if (++spins > a.spin_limit) {
+      if (lane == 0) atomicOr(&a.ctl->err, ERR_TIMEOUT);
+      return false;
+    }
+    __nanosleep(spins < 8 ? 32 : 256);
+  }
+  __syncwarp();
+  const unsigned long long vmask = (1ull << 38) - 1;
+  excl = __shfl_sync(0xffffffffu, w, 0) & vmask;
+  total = (unsigned)((__shfl_sync(0xffffffffu, w, 1) & vmask) - excl);
+  return true;
+}
+
+// ------------------------------------------------------------------------------------
+// Records from face codes. A warp writes the records of up to 32 consecutive faces: lane l builds
+// the record of its face in the warp's staging buffer, then the lanes copy the buffer to the
+// output in 16-byte units, so that every store covers whole lines. Emission is short of warps
+// as long as it waits for generation, so its time is the instructions of a batch: about 65
+// this way. Building each 16-byte unit in the lane that stores it (no buffer; a shuffle, a
+// table entry and the translation per unit) took 215, or 670 for instances, and sending the
+// buffer with a TMA bulk copy waits about a microsecond for the copy to have read it.
+// ------------------------------------------------------------------------------------
+
+constexpr int kEmitThreads = 256;
+
+// Translations of a chunk: local coordinate q_c of byte c of a face code -> world coordinate
+// o_c + q_c as a float, rounded once. Origins below 2^23 - 64 in size take a shorter way with the
+// same result: the byte in the low mantissa of 2^23 is exact, and so is every sum here.
+struct Origin {
+  int o[3];
+  float f[3];  // (float)o - 2^23
+  bool small;
+  __device__ Origin(vox_chunk_coord c, int n) : o{c.x * n, c.y * n, c.z * n} {
+    constexpr int kLim = (1 << 23) - 64;
+    small = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      small = small && o[k] > -kLim && o[k] < kLim;
+      f[k] = (float)o[k] - 8388608.0f;
+    }
+  }
+  template <bool kSmall>
+  __device__ __forceinline__ float at(uint32_t q, int k) const {
+    return kSmall ? __uint_as_float(__byte_perm(q, 0x4B000000u, 0x7440u | (unsigned)k)) + f[k]
+                  : (float)(o[k] + (int)((q >> (8 * k)) & 255u));
+  }
+};
+
+template <int LAYOUT>
+struct FaceStore;
+
+template <>
+struct FaceStore<VOX_LAYOUT_VERTEX> {
+  static constexpr int kTableBytes = 6 * 64;         // per direction 12 corner coordinates, face
+  static constexpr int kBufBytes = kWarpBatch * 96;  // a warp's buffer
+  const float4* table;
+  float4* buf;
+  int lane;
+
+  // Fills the table (all threads; the caller synchronises) and sets up the lane.
+  __device__ void init(unsigned char* smem, unsigned char* bufs, const TablesDev& tab) {
+    table = reinterpret_cast<const float4*>(smem);
+    lane = threadIdx.x & 31;
+    buf = reinterpret_cast<float4*>(bufs + (threadIdx.x >> 5) * kBufBytes);
+    if (threadIdx.x < 6 * 13) {
+      const int d = threadIdx.x / 13, k = threadIdx.x % 13;
+      reinterpret_cast<float*>(smem)[d * 16 + k] =
+          k < 12 ? (&tab.corner[d][0][0])[k] : __uint_as_float(tab.slot[d]);
+    }
+  }
+
+  // Writes nw faces (chunk-local indices first, first + 1, ...) at global face g.
+  template <bool kSmall>
+  __device__ __forceinline__ void batch(uint32_t q, int nw, uint32_t first, const Origin& org,
+                                        unsigned long long g, void* out0, void* out1) const {
+    const float4* C = table + (q >> 24) * 4u;
+    const float4 c0 = C[0], c1 = C[1], c2 = C[2];
+    const float face = C[3].x;
+    const float tx = org.at<kSmall>(q, 0), ty = org.at<kSmall>(q, 1), tz = org.at<kSmall>(q, 2);
+    float4* v = buf + lane * 6;
+    __syncwarp();  // the last batch has been copied out
+    // position, tex coords (0,0) (1,0) (0,1) (1,1) (src/quad.rs:66-87) and face, 6 words a vertex
+    v[0] = make_float4(c0.x + tx, c0.y + ty, c0.z + tz, 0.0f);
+    v[1] = make_float4(0.0f, face, c0.w + tx, c1.x + ty);
+    v[2] = make_float4(c1.y + tz, 1.0f, 0.0f, face);
+    v[3] = make_float4(c1.z + tx, c1.w + ty, c2.x + tz, 0.0f);
+    v[4] = make_float4(1.0f, face, c2.y + tx, c2.z + ty);
+    v[5] = make_float4(c2.w + tz, 1.0f, 1.0f, face);
+    __syncwarp();
+    float4* o = reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(out0) + g * 96ull) + lane;
+    const int units = nw * 6;
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      if (32 * k + lane < units) o[32 * k] = buf[32 * k + lane];
+    // indices 4 f + {0, 2, 1, 3, 1, 2}: 8-byte pair j of face u / 3
+    uint2* x = reinterpret_cast<uint2*>(reinterpret_cast<unsigned char*>(out1) + g * 24ull) + lane;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int u = 32 * k + lane, f = u / 3, j = u - 3 * f;
+      const uint32_t b = 4u * (first + (uint32_t)f);
+      if (f < nw) x[32 * k] = make_uint2(b + (j == 0 ? 0u : 1u), b + (j == 1 ? 3u : 2u));
+    }
+  }
+};
+
+template <>
+struct FaceStore<VOX_LAYOUT_INSTANCED> {
+  static constexpr int kTableBytes = 6 * 80;  // per direction the 17 words of a record
+  static constexpr int kBufBytes = kWarpBatch * 68;
+  const float* table;
+  float* buf;
+  int lane;
+
+  __device__ void init(unsigned char* smem, unsigned char* bufs, const TablesDev& tab) {
+    table = reinterpret_cast<const float*>(smem);
+    lane = threadIdx.x & 31;
+    buf = reinterpret_cast<float*>(bufs + (threadIdx.x >> 5) * kBufBytes);
+    if (threadIdx.x < 6 * 17) {
+      const int d = threadIdx.x / 17, w = threadIdx.x % 17, c = w >> 2, r = w & 3;
+      float v;
+      if (w == 16) v = __uint_as_float(tab.tex[d]);
+      else if (c == 3) v = 1.0f;
+      else v = r == 3 ? tab.row3[d][c] : tab.part[d][r][c];
+      reinterpret_cast<float*>(smem)[d * 20 + w] = v;
+    }
+  }
+
+  template <bool kSmall>
+  __device__ __forceinline__ void batch(uint32_t q, int nw, uint32_t, const Origin& org,
+                                        unsigned long long g, void* out0, void*) const {
+    const float4* M = reinterpret_cast<const float4*>(table + (q >> 24) * 20u);
+    const float tx = org.at<kSmall>(q, 0), ty = org.at<kSmall>(q, 1), tz = org.at<kSmall>(q, 2);
+    const float z0 = tx * 0.0f, z1 = ty * 0.0f, z2 = tz * 0.0f;
+    const float tex = table[(q >> 24) * 20u + 16u];
+    float* v = buf + lane * 17;
+    __syncwarp();  // the last batch has been copied out
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {  // column c of the matrix: t_r * 0 decides the sign of a zero
+      const float4 m = M[c];
+      v[4 * c + 0] = m.x + z0;
+      v[4 * c + 1] = m.y + z1;
+      v[4 * c + 2] = m.z + z2;
+      v[4 * c + 3] = m.w;
+    }
+    v[12] = tx;
+    v[13] = ty;
+    v[14] = tz;
+    v[15] = 1.0f;
+    v[16] = tex;
+    __syncwarp();
+    unsigned char* o = reinterpret_cast<unsigned char*>(out0) + g * 68ull;
+    if (((unsigned)g & 3u) == 0u) {  // 16-byte units, and the words of the last up to 3 faces
+      const int units = nw * 17 >> 2;
+#pragma unroll
+      for (int k = 0; k < 5; ++k)
+        if (32 * k + lane < units)
+          reinterpret_cast<float4*>(o)[32 * k + lane] = reinterpret_cast<const float4*>(buf)[32 * k + lane];
+      if (lane < (nw * 17 & 3))
+        reinterpret_cast<float*>(o)[4 * units + lane] = buf[4 * units + lane];
+    } else {
+      for (int k = lane; k < nw * 17; k += 32) reinterpret_cast<float*>(o)[k] = buf[k];
+    }
+  }
+};
+
+template <int N, int LAYOUT>
+__global__ void __launch_bounds__(kEmitThreads, 4)
+k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesDev tab) {
+  using S = ListSlot<N>;
+  constexpr unsigned kLine = line_faces<LAYOUT>();
+  using Store = FaceStore<LAYOUT>;
+  __shared__ __align__(16) unsigned char s_table[Store::kTableBytes];
+  __shared__ __align__(16) unsigned char s_bufs[kEmitThreads / 32 * Store::kBufBytes];
+  __shared__ uint32_t s_lists[kEmitThreads / 32 * kWarpFaces];
+  __shared__ unsigned long long s_base0;
+  __shared__ unsigned s_epoch;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  Store store;
+  store.init(s_table, s_bufs, tab);
+  if (t == 0) {
+    s_epoch = ld_relaxed_u32(&a.ctl->epoch);
+    s_base0 = launch_base(a);
+  }
+  __syncthreads();
+  const unsigned epoch = s_epoch;
+  const unsigned long long base0 = s_base0;
+  bool ok = true;
+  if (warp == 0) {  // scan items, in ticket order: a running warp holds every smaller ticket
+    const unsigned scans = ((unsigned)a.n + kGroup - 1u) / kGroup;
+    while (ok) {
+      unsigned g = 0;
+      if (lane == 0) g = atomicAdd(&a.ctl->next_scan, 1u);
+      g = __shfl_sync(0xffffffffu, g, 0);
+      if (g >= scans) break;
+      ok = scan_group(a, epoch, (int)g, base0);
+    }
+  }
+  // Emission items: part k % 2^split of chunk k >> split, dealt out to the warps of the grid in
+  // chunk order.
+  const unsigned parts = 1u << a.split;
+  const unsigned long long items = (unsigned long long)a.n << a.split;
+  for (unsigned long long k = (unsigned long long)blockIdx.x * (kEmitThreads / 32) + warp;
+       ok && k < items; k += (unsigned long long)gridDim.x * (kEmitThreads / 32)) {
+    const int i = (int)(k >> a.split);
+    const unsigned part = (unsigned)k & (parts - 1u);
+    const vox_chunk_coord c = a.coords[i];
+    unsigned long long g0;
+    unsigned total;
+    ok = chunk_offset(a, epoch, i, g0, total);
+    if (!ok || total == 0u) continue;
+    g0 += base0;
+    const Origin org(c, N);
+    auto send = [&](uint32_t q, int nw, uint32_t first, unsigned long long g) {
+      if (org.small) store.template batch<true>(q, nw, first, org, g, a.out0, a.out1);
+      else store.template batch<false>(q, nw, first, org, g, a.out0, a.out1);
+    };
+    unsigned char* src = reinterpret_cast<unsigned char*>(a.scratch) + (unsigned long long)i * S::kBytes;
+    if (total <= S::kCap) {
+      // the output lines that the chunk touches, cut evenly over the parts
+      const uint32_t* codes = reinterpret_cast<const uint32_t*>(src);
+      const unsigned phase = (unsigned)(g0 & (unsigned long long)(kLine - 1u));
+      const unsigned lines = (phase + total + kLine - 1u) / kLine;
+      const unsigned la = (unsigned)(((unsigned long long)lines * part) >> a.split);
+      const unsigned lb = (unsigned)(((unsigned long long)lines * (part + 1u)) >> a.split);
+      if (la == lb) continue;
+      const int lo = la == 0u ? 0 : (int)(la * kLine - phase);
+      const int hi = (int)min(total, lb * kLine - phase);
+      int cnt = batch_faces<LAYOUT>(g0 + (unsigned)lo, hi - lo);
+      uint32_t q = lane < cnt ? __ldcg(codes + lo + lane) : 0u;
+      for (int r = lo; r < hi;) {
+        const unsigned long long g = g0 + (unsigned)r;
+        const int r2 = r + cnt;
+        const int cnt2 = r2 < hi ? batch_faces<LAYOUT>(g0 + (unsigned)r2, hi - r2) : 0;
+        const uint32_t q2 = lane < cnt2 ? __ldcg(codes + r2 + lane) : 0u;  // the next batch
+        const int nw = faces_in(g, cnt, a.cap);
+        if (nw == 0) break;
+        send(q, nw, (uint32_t)r, g);
+        r = r2;
+        cnt = cnt2;
+        q = q2;
+      }
+    } else {  // no list: compaction from the spilled chunk state
+      ChunkSmem<N, LAYOUT> d;
+      d.occ = reinterpret_cast<typename Shape<N>::RowT*>(src);
+      d.halo = reinterpret_cast<typename Shape<N>::RowT*>(src + S::P::kOcc);
+      d.rows = reinterpret_cast<uint32_t*>(src + S::P::kOcc + S::P::kHalo);
+      d.nz = reinterpret_cast<uint16_t*>(src + S::kNzOff);
+      d.vlist = reinterpret_cast<uint16_t*>(src + S::kVlOff);
+      d.misc = reinterpret_cast<int*>(src + S::kMiscOff);
+      d.lists = s_lists;
+      emit_runs<N, LAYOUT>(d, 0, emit_elems(d), (int)part, (int)parts, g0,
+                           [&](const uint32_t* list, int nf, uint32_t first) {
+        for (int r = 0, cnt = 0; r < nf; r += cnt) {
+          const unsigned long long g = g0 + first + (unsigned)r;
+          cnt = batch_faces<LAYOUT>(g, nf - r);
+          const int nw = faces_in(g, cnt, a.cap);
+          if (nw == 0) continue;
+          send(lane < nw ? list[r + lane] : 0u, nw, first + (uint32_t)r, g);
+        }
+        __syncwarp();
+      });
+    }
+  }
+  // The last CTA to finish resets the scan tickets and advances the epoch: every chunk of the
+  // launch is published and emitted by then.
+  __syncthreads();
+  if (t == 0) {
+    __threadfence();
+    if (atomicAdd(&a.ctl->done, 1u) == gridDim.x - 1u) {
+      a.ctl->done = 0u;
+      a.ctl->next_scan = 0u;
+      a.ctl->epoch = epoch + 1u;
+    }
+  }
+  // the generation launch has completed too before this one does
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+}  // namespace vox

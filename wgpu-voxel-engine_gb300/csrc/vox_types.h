@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <type_traits>
+#include <vector_types.h>
 
 #include "voxgpu.h"
 
@@ -39,6 +40,13 @@ struct TablesDev {
   float grad[16][4];      // gradient coefficients (gx, gy, gz, 0) of hash & 15
 };
 
+// Words of the look-back states of a launch of n chunks: one per chunk, then one per group of
+// kStateGroup chunks (see scan_group).
+constexpr unsigned long long kStateGroup = 32;
+constexpr unsigned long long state_words(unsigned long long n) {
+  return n + (n + kStateGroup - 1) / kStateGroup;
+}
+
 struct BatchCtl {
   unsigned int next;       // work-queue ticket; reset to 0 by the last CTA of a launch
   unsigned int epoch;      // look-back state tag; advanced by the last CTA of a launch
@@ -47,8 +55,11 @@ struct BatchCtl {
   unsigned int bar_gen;    // grid barrier: generation, advanced by the last arriver
   unsigned int scan_flag;  // phased kernel: the generation whose offset scan is complete
   unsigned int done;       // CTAs finished in a launch that mirrors its status (reset by the last)
-  unsigned int pad;
+  unsigned int next_scan;  // k_emit_lists: scan tickets (reset by its last CTA)
 };
+
+// Gradients of the hashed 2-D lattice corners: entry A is the gradient (gx, gy) of p[p[A]].
+constexpr int kGrad2 = 512;
 
 struct MeshArgs {
   int n;
@@ -66,9 +77,10 @@ struct MeshArgs {
   void* out1;
   unsigned long long cap;
   unsigned long long* face_offsets;  // n + 1 entries (single chunk: the count at [0])
-  unsigned long long* state;         // look-back states, n entries
+  unsigned long long* state;         // look-back states: chunks, then groups (see state_words)
   BatchCtl* ctl;
   const TablesDev* tables;
+  const float2* grad2;               // kGrad2 entries, or null (heightmap generation)
   GenDev gen;
   int full6;
   int stage_faces;                   // faces per staging window (0: direct global stores)

@@ -9,7 +9,7 @@ memory comes from torch (plumbing only); every launch goes through the C ABI.
 """
 from __future__ import annotations
 
-from . import VOX_OK, VOX_ERR_CAPACITY, VoxError
+from . import GEN_BERNOULLI, SCHEDULE_OVERLAP, VOX_OK, VOX_ERR_CAPACITY, VoxError
 
 
 class BatchRun:
@@ -17,7 +17,8 @@ class BatchRun:
 
     After construction: `offsets` (n + 1 int64 on the device, chunk i's first face and the
     total), `out0` / `out1` (uint8 device tensors of total * bytes-per-face), `total_faces`,
-    `tuning` (the context's launch shape as a dict) and, with graph=True, one captured graph
+    `tuning` (the context's launch shape as a dict), `launches_per_step` (batch launches, with the
+    staged-halo ones) and `kernels_per_step`, and, with graph=True, one captured graph
     holding every slab launch of the batch."""
 
     def __init__(self, ctx, coords, masks=None, index_base: int = 0, autotune: bool = False,
@@ -57,6 +58,10 @@ class BatchRun:
             # staged halos: coordinate map (with the identity slots), neighbour lookup,
             # generation of the batch and (with neighbour masks) of the halo planes outside it
             self.launches_per_step += 3 + (1 if masks is not None else 0)
+        # the overlap schedule's batch launch is two kernels: face lists, then records (random
+        # voxels, unless they are staged in a pool: one kernel)
+        two = t.schedule == SCHEDULE_OVERLAP and (ctx.cfg.gen.kind != GEN_BERNOULLI or t.halo_staging)
+        self.kernels_per_step = self.launches_per_step + ((n + slab - 1) // slab if two else 0)
         self.graph = (ctx.capture_graph(self.d_coords, self.d_mask, n, self.out0, self.out1,
                                         self.cap, self.offsets, chunk_index_base=index_base)
                       if graph else None)
