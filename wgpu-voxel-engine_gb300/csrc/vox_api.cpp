@@ -711,9 +711,8 @@ int vox_ctx_create(const vox_config* cfg, void* stream, vox_ctx** out) {
           (st = prepare_kernel(ctx, ctx->ks->phased[gm][layout][t], ctx->max_smem_optin)) != VOX_OK ||
           (st = prepare_kernel(ctx, ctx->ks->overlap[gm][layout][t], ctx->max_smem_optin)) != VOX_OK)
         return cleanup(st);
-  for (int t = 0; t < 2; ++t)
-    if ((st = prepare_kernel(ctx, ctx->ks->single[layout][t], ctx->max_smem_optin)) != VOX_OK)
-      return cleanup(st);
+  if ((st = prepare_kernel(ctx, ctx->ks->single[layout], ctx->ks->single_smem[layout])) != VOX_OK)
+    return cleanup(st);
   const int gsmem = ctx->ks->smem_total(VOX_LAYOUT_VERTEX, ctx->ks->gen_threads, 0);
   for (int gm = 1; gm < 4; ++gm)
     if ((st = prepare_kernel(ctx, ctx->ks->generate[gm], gsmem)) != VOX_OK ||
@@ -890,11 +889,10 @@ int vox_mesh(vox_ctx* ctx, const uint32_t* d_occ, const uint32_t* const d_nbr[6]
   a.out1 = d_out1;
   a.cap = cap_faces;
   a.face_offsets = reinterpret_cast<unsigned long long*>(d_face_count);
-  void* params[] = {&a};
+  void* params[] = {&a, &ctx->h_tables};
   const int layout = ctx->cfg.layout;
-  return launch(ctx, ctx->ks->single[layout][ctx->topt], 1, ctx->ks->threads[ctx->topt],
-                ctx->ks->smem_total(layout, ctx->ks->threads[ctx->topt], ctx->stage_faces),
-                params);
+  return launch(ctx, ctx->ks->single[layout], ctx->ks->single_ctas, ctx->ks->single_threads,
+                ctx->ks->single_smem[layout], params);
 }
 
 int vox_mesh_batch(vox_ctx* ctx, const uint32_t* d_occ_pool, int32_t pool_slots,

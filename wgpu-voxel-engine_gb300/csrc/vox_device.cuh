@@ -1289,44 +1289,53 @@ __device__ void gen_chunk(ChunkSmem<N, LAYOUT>& s, const GenDev& g, vox_chunk_co
 }
 
 // Occupancy from global memory: own rows copied; halo rows taken from the neighbours'
-// boundary planes (nbr[d] == nullptr: not loaded, zero halo).
-template <int N, int LAYOUT>
-__device__ void load_chunk(ChunkSmem<N, LAYOUT>& s, const uint32_t* self,
-                           const uint32_t* const nbr[6], unsigned use_mask) {
-  using RowT = typename Shape<N>::RowT;
+// boundary planes (nbr[d] == nullptr: not loaded, zero halo). Every thread issues all its loads
+// before it uses one, so the chunk costs one memory latency instead of one per plane.
+template <int N, int LAYOUT, int T>
+__device__ __forceinline__ void load_chunk(ChunkSmem<N, LAYOUT>& s, const uint32_t* self,
+                                           const uint32_t* const nbr[6], unsigned use_mask) {
   constexpr int W = Shape<N>::W;
+  constexpr int kOwn = N * N * W / T, kPlane = N * N / T, kRow = N * W;
+  static_assert(kPlane >= 1 && kPlane * T == N * N, "planes must split evenly over threads");
+  constexpr int kMost = N > 32 ? 4 : kOwn;  // own words in flight (64^3: in turns)
   uint32_t* occw = reinterpret_cast<uint32_t*>(s.occ);
-  for (int i = threadIdx.x; i < N * N * W; i += blockDim.x) occw[i] = __ldg(self + i);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   uint32_t* halow = reinterpret_cast<uint32_t*>(s.halo);
-  for (int h = 0; h < 6; ++h) {
+  const int t = threadIdx.x;
+  uint32_t own[kMost], px[2][kPlane], pr = 0u;
+#pragma unroll
+  for (int k = 0; k < kMost; ++k) own[k] = __ldg(self + t + k * T);
+  // x planes: bit (N - 1) (h = 0) or bit 0 (h = 1) of the neighbour's row (y, z)
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
     const uint32_t* nb = ((use_mask >> h) & 1u) ? nbr[h] : nullptr;
-    if (!nb) {
-      for (int i = threadIdx.x; i < N; i += blockDim.x) s.halo[h * N + i] = (RowT)0;
-      continue;
-    }
-    if (h <= 1) {
-      // bit (N-1) (h = 0) or bit 0 (h = 1) of the neighbour's row (y, z), gathered over z.
-      const int bx = h == 0 ? N - 1 : 0;
-      for (int base = warp * 32; base < N * N; base += nwarps * 32) {
-        const int e = base + lane;
-        const int y = e / N, z = e % N;
-        const uint32_t w = __ldg(nb + (y * N + z) * W + (bx >> 5));
-        store_ballot<N>(halow + h * N * W, e, ((w >> (bx & 31)) & 1u) != 0u);
-      }
-    } else {
-      // whole rows: -z: (y, N-1); +z: (y, 0); -y: (N-1, z); +y: (0, z).
-      for (int i = threadIdx.x; i < N * W; i += blockDim.x) {
-        const int a = i / W, w = i % W;
-        int r;
-        if (h == 2) r = a * N + (N - 1);
-        else if (h == 3) r = a * N;
-        else if (h == 4) r = (N - 1) * N + a;
-        else r = a;
-        halow[(h * N + a) * W + w] = __ldg(nb + r * W + w);
-      }
-    }
+    constexpr int kLast = (N - 1) >> 5;
+#pragma unroll
+    for (int k = 0; k < kPlane; ++k)
+      px[h][k] = nb ? __ldg(nb + (t + k * T) * W + (h == 0 ? kLast : 0)) >> (h == 0 ? (N - 1) & 31 : 0) : 0u;
   }
+  // whole rows: -z: (y, N-1); +z: (y, 0); -y: (N-1, z); +y: (0, z)
+  auto row_word = [&](int i) {
+    const int h = 2 + i / kRow, a = (i % kRow) / W, w = i % W;
+    const uint32_t* nb = ((use_mask >> h) & 1u) ? nbr[h] : nullptr;
+    const int r = h == 2 ? a * N + (N - 1) : (h == 3 ? a * N : (h == 4 ? (N - 1) * N + a : a));
+    return nb ? __ldg(nb + r * W + w) : 0u;
+  };
+  if (t < 4 * kRow) pr = row_word(t);
+#pragma unroll
+  for (int k = 0; k < kMost; ++k) occw[t + k * T] = own[k];
+  for (int k = kMost; k < kOwn; k += kMost) {
+#pragma unroll
+    for (int j = 0; j < kMost; ++j) own[j] = __ldg(self + t + (k + j) * T);
+#pragma unroll
+    for (int j = 0; j < kMost; ++j) occw[t + (k + j) * T] = own[j];
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int k = 0; k < kPlane; ++k)
+      store_ballot<N>(halow + h * N * W, t + k * T, (px[h][k] & 1u) != 0u);
+  if (t < 4 * kRow) halow[2 * kRow + t] = pr;
+  for (int i = t + T; i < 4 * kRow; i += T) halow[2 * kRow + i] = row_word(i);
   __syncthreads();
 }
 
@@ -2182,7 +2191,7 @@ __device__ __forceinline__ void prepare_chunk(ChunkSmem<N, LAYOUT>& s, const Mes
     if (bad && threadIdx.x == 0) atomicOr(&a.ctl->err, ERR_BAD_INPUT);
     // An out-of-range slot reads slot 0 instead (the call then reports VOX_ERR_INVALID).
     const int sl = (slot >= 0 && slot < a.pool_slots) ? slot : 0;
-    load_chunk<N, LAYOUT>(s, a.occ_pool + (unsigned long long)sl * words, nb, use);
+    load_chunk<N, LAYOUT, T>(s, a.occ_pool + (unsigned long long)sl * words, nb, use);
   } else {
     unsigned m = a.nbr_mask ? a.nbr_mask[i] : 0u;
     if (GM == GM_BERNOULLI) m = 0u;
@@ -2698,31 +2707,6 @@ k_mesh_batch_overlap(const __grid_constant__ MeshArgs a, const __grid_constant__
   }
   if ((t & 31) == 0) bulk_wait_all();  // every lane 0 issued bulk copies
   finish_launch(a);
-}
-
-// Plain per-chunk mesher: one chunk, one CTA, one launch (no queue, no look-back).
-template <int N, int LAYOUT, int T>
-__global__ void __launch_bounds__(T)
-k_mesh_single(MeshArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  ChunkSmem<N, LAYOUT> s;
-  s.carve(smem_raw);
-  load_tables<N, LAYOUT>(s, a.tables);
-  unsigned use = 0;
-  for (int d = 0; d < 6; ++d)
-    if (a.occ_nbr[d] && (d < 4 || a.full6)) use |= 1u << d;
-  load_chunk<N, LAYOUT>(s, a.occ_self, a.occ_nbr, use);
-  const uint32_t total = count_and_scan<N, LAYOUT, T>(s);
-  if (threadIdx.x == 0) {
-    a.face_offsets[0] = total;
-    if ((unsigned long long)total > a.cap) atomicOr(&a.ctl->err, ERR_CAPACITY);
-  }
-  if (a.stage_faces > 0)
-    emit_chunk<N, LAYOUT>(s, a.coord_single, 0ull, a.cap, a.out0, a.out1, a.stage_faces / kWarpBatch,
-                          a.lane_flush != 0, 0, emit_elems(s), threadIdx.x >> 5, T / 32);
-  else emit_chunk_direct<N, LAYOUT>(s, a.coord_single, 0ull, a.cap, a.out0, a.out1, 0, emit_elems(s),
-                                        threadIdx.x >> 5, T / 32);
-  if ((threadIdx.x & 31) == 0) bulk_wait_all();
 }
 
 // Register budget of k_generate as resident CTAs per SM: 64 registers a thread for the 3-D

@@ -47,10 +47,12 @@ static KernelSet make_kernel_set() {
   fill_batch<N, GM_DENSITY, VOX_LAYOUT_INSTANCED>(k);
   fill_batch<N, GM_BERNOULLI, VOX_LAYOUT_VERTEX>(k);
   fill_batch<N, GM_BERNOULLI, VOX_LAYOUT_INSTANCED>(k);
-  k.single[0][0] = (const void*)k_mesh_single<N, VOX_LAYOUT_VERTEX, Shape<N>::T0>;
-  k.single[0][1] = (const void*)k_mesh_single<N, VOX_LAYOUT_VERTEX, Shape<N>::T1>;
-  k.single[1][0] = (const void*)k_mesh_single<N, VOX_LAYOUT_INSTANCED, Shape<N>::T0>;
-  k.single[1][1] = (const void*)k_mesh_single<N, VOX_LAYOUT_INSTANCED, Shape<N>::T1>;
+  k.single[VOX_LAYOUT_VERTEX] = (const void*)k_mesh_single<N, VOX_LAYOUT_VERTEX>;
+  k.single[VOX_LAYOUT_INSTANCED] = (const void*)k_mesh_single<N, VOX_LAYOUT_INSTANCED>;
+  k.single_smem[VOX_LAYOUT_VERTEX] = single_smem<N, VOX_LAYOUT_VERTEX>();
+  k.single_smem[VOX_LAYOUT_INSTANCED] = single_smem<N, VOX_LAYOUT_INSTANCED>();
+  k.single_threads = single_threads<N>();
+  k.single_ctas = single_ctas<N>();
   fill_lists<N, GM_OCC>(k);
   fill_lists<N, GM_HEIGHT>(k);
   fill_lists<N, GM_DENSITY>(k);

@@ -13,7 +13,8 @@ struct KernelSet {
   const void* batch[4][2][2];   // k_mesh_batch<N, gen mode, layout, threads[t]>
   const void* phased[4][2][2];  // k_mesh_batch_phased<N, gen mode, layout, threads[t]>
   const void* overlap[4][2][2]; // k_mesh_batch_overlap<N, gen mode, layout, threads[t]>
-  const void* single[2][2];     // k_mesh_single<N, layout, threads[t]>
+  const void* single[2];        // k_mesh_single<N, layout>
+  int single_smem[2], single_threads, single_ctas;
   const void* generate[4];      // k_generate<N, gen mode, gen_threads> (index 0 unused)
   const void* generate_planes[4]; // k_generate_planes<N, gen mode, gen_threads> (height, density)
   // the list launches (vox_lists.cuh); none for Bernoulli chunks, which have too many faces

@@ -55,6 +55,16 @@ struct ListSmem {
                                   : GM == GM_HEIGHT ? (N > 32 ? P::kHeight : kGrad2 * 8)
                                                     : 0;
   static constexpr int kBytes = kRowsOff + (kScratch > kLists + 256 ? kScratch : kLists + 256);
+  // The generator's scratch is at lists(base); the count's is behind the lists.
+  __device__ static unsigned char* lists(unsigned char* base) { return base + kRowsOff; }
+  __device__ static void carve(ChunkSmem<N, VOX_LAYOUT_VERTEX>& s, unsigned char* base) {
+    s.carve(base, 0);
+    s.misc = reinterpret_cast<int*>(base + P::kTables + P::kOcc + P::kHalo);
+    s.rows = reinterpret_cast<uint32_t*>(lists(base));
+    s.nz = reinterpret_cast<uint16_t*>(lists(base) + P::kRows);
+    s.vlist = reinterpret_cast<uint16_t*>(lists(base) + P::kRows + P::kNz);
+    s.scratch_at(lists(base));
+  }
 };
 
 // Resident CTAs per SM that k_list_chunks is compiled for (its register budget): 64 registers
@@ -76,13 +86,8 @@ k_list_chunks(const __grid_constant__ MeshArgs a, const __grid_constant__ Tables
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using M = ListSmem<N, GM>;
   ChunkSmem<N, VOX_LAYOUT_VERTEX> s;
-  s.carve(smem_raw, 0);
-  s.misc = reinterpret_cast<int*>(smem_raw + P::kTables + P::kOcc + P::kHalo);
-  unsigned char* const lists = smem_raw + M::kRowsOff;
-  s.rows = reinterpret_cast<uint32_t*>(lists);
-  s.nz = reinterpret_cast<uint16_t*>(lists + P::kRows);
-  s.vlist = reinterpret_cast<uint16_t*>(lists + P::kRows + P::kNz);
-  s.scratch_at(lists);
+  M::carve(s, smem_raw);
+  unsigned char* const lists = M::lists(smem_raw);
   const int i = blockIdx.x, t = threadIdx.x;
   unsigned epoch = 0;
   if (t == 0) epoch = ld_relaxed_u32(&a.ctl->epoch);
@@ -244,8 +249,8 @@ struct FaceStore<VOX_LAYOUT_VERTEX> {
     table = reinterpret_cast<const float4*>(smem);
     lane = threadIdx.x & 31;
     buf = reinterpret_cast<float4*>(bufs + (threadIdx.x >> 5) * kBufBytes);
-    if (threadIdx.x < 6 * 13) {
-      const int d = threadIdx.x / 13, k = threadIdx.x % 13;
+    for (int i = threadIdx.x; i < 6 * 13; i += blockDim.x) {
+      const int d = i / 13, k = i % 13;
       reinterpret_cast<float*>(smem)[d * 16 + k] =
           k < 12 ? (&tab.corner[d][0][0])[k] : __uint_as_float(tab.slot[d]);
     }
@@ -297,8 +302,8 @@ struct FaceStore<VOX_LAYOUT_INSTANCED> {
     table = reinterpret_cast<const float*>(smem);
     lane = threadIdx.x & 31;
     buf = reinterpret_cast<float*>(bufs + (threadIdx.x >> 5) * kBufBytes);
-    if (threadIdx.x < 6 * 17) {
-      const int d = threadIdx.x / 17, w = threadIdx.x % 17, c = w >> 2, r = w & 3;
+    for (int i = threadIdx.x; i < 6 * 17; i += blockDim.x) {
+      const int d = i / 17, w = i % 17, c = w >> 2, r = w & 3;
       float v;
       if (w == 16) v = __uint_as_float(tab.tex[d]);
       else if (c == 3) v = 1.0f;
@@ -456,6 +461,67 @@ k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
   }
   // the generation launch has completed too before this one does
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// ------------------------------------------------------------------------------------
+// Plain per-chunk mesher: one chunk, one launch (no queue, no look-back). One CTA used to do
+// it all, so a chunk's emission ran on one SM of 152. Now single_ctas CTAs each load and count
+// the whole chunk (redundant, but the GPU has nothing else to do and the counts need no
+// exchange) and emit their part of it: a few groups of 32 face voxels a warp. A call on a
+// terrain chunk of 64^3 238 -> 17.8 us, a cave chunk of 64^3 as instances 139 -> 22.4 us; from
+// 32^3 down a call is bound by the caller (16 us through Python either way; waiting for one
+// chunk of 32^3 takes about 5 us less).
+// ------------------------------------------------------------------------------------
+
+template <int N>
+__host__ __device__ constexpr int single_threads() {
+  return N == 8 ? 64 : (N == 16 ? 256 : (N == 32 ? 512 : 1024));
+}
+template <int N>
+__host__ __device__ constexpr int single_ctas() { return N == 8 ? 1 : (N == 16 ? 2 : (N == 32 ? 8 : 64)); }
+template <int N, int LAYOUT>
+__host__ __device__ constexpr int single_smem() {
+  return ListSmem<N, GM_OCC>::kBytes +
+         single_threads<N>() / 32 * (kWarpFaces * 4 + FaceStore<LAYOUT>::kBufBytes);
+}
+
+template <int N, int LAYOUT>
+__global__ void __launch_bounds__(single_threads<N>())
+k_mesh_single(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesDev tab) {
+  using M = ListSmem<N, GM_OCC>;
+  constexpr int T = single_threads<N>();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(16) unsigned char s_table[FaceStore<LAYOUT>::kTableBytes];
+  ChunkSmem<N, VOX_LAYOUT_VERTEX> s;
+  M::carve(s, smem_raw);
+  s.lists = reinterpret_cast<uint32_t*>(smem_raw + M::kBytes);
+  const int t = threadIdx.x, lane = t & 31;
+  FaceStore<LAYOUT> store;
+  store.init(s_table, smem_raw + M::kBytes + T / 32 * kWarpFaces * 4, tab);
+  unsigned use = 0;
+  for (int d = 0; d < 6; ++d)
+    if (a.occ_nbr[d] && (d < 4 || a.full6)) use |= 1u << d;
+  load_chunk<N, VOX_LAYOUT_VERTEX, T>(s, a.occ_self, a.occ_nbr, use);
+  s.stage = smem_raw + M::kRowsOff + M::kLists;
+  const uint32_t total = count_and_scan<N, VOX_LAYOUT_VERTEX, T>(s);
+  if (blockIdx.x == 0 && t == 0) {
+    a.face_offsets[0] = total;
+    if ((unsigned long long)total > a.cap) atomicOr(&a.ctl->err, ERR_CAPACITY);
+  }
+  const Origin org(a.coord_single, N);
+  emit_runs<N, LAYOUT>(s, 0, emit_elems(s), (int)blockIdx.x * (T / 32) + (t >> 5),
+                       (int)gridDim.x * (T / 32), 0ull, [&](const uint32_t* list, int nf, uint32_t first) {
+    for (int r = 0, cnt = 0; r < nf; r += cnt) {
+      const unsigned long long g = first + (unsigned)r;
+      cnt = batch_faces<LAYOUT>(g, nf - r);
+      const int nw = faces_in(g, cnt, a.cap);
+      if (nw == 0) continue;
+      const uint32_t q = lane < nw ? list[r + lane] : 0u;
+      if (org.small) store.template batch<true>(q, nw, (uint32_t)g, org, g, a.out0, a.out1);
+      else store.template batch<false>(q, nw, (uint32_t)g, org, g, a.out0, a.out1);
+    }
+    __syncwarp();
+  });
 }
 
 }  // namespace vox
