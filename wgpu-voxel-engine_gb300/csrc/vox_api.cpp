@@ -15,6 +15,7 @@
 
 #include "voxgpu.h"
 #include "vox_kernels.h"
+#include "vox_launch.h"
 #include "vox_tables.h"
 #include "vox_trace.h"
 #include "vox_types.h"
@@ -396,18 +397,9 @@ int issue_lists(vox_ctx* ctx, MeshArgs& a, int gm, cudaStream_t stream) {
   VOX_CUDA(ctx, cudaLaunchKernel(ks.list[gm][big], dim3(a.n), dim3(ks.list_threads[big]), params,
                                  (size_t)ks.list_smem[gm], stream),
            "cudaLaunchKernel(lists)");
-  cudaLaunchAttribute attr;
-  std::memset(&attr, 0, sizeof attr);
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg;
-  std::memset(&cfg, 0, sizeof cfg);
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(ks.emit_threads);
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  VOX_CUDA(ctx, cudaLaunchKernelExC(&cfg, ks.emit[ctx->cfg.layout], params), "cudaLaunchKernelExC(emission)");
+  VOX_CUDA(ctx, launch_dependent(ks.emit[ctx->cfg.layout], dim3(grid), dim3(ks.emit_threads), params, 0,
+                                 stream),
+           "cudaLaunchKernelExC(emission)");
   return VOX_OK;
 }
 

@@ -19,6 +19,7 @@
 #pragma once
 
 #include "vox_device.cuh"
+#include "vox_launch.h"
 
 namespace vox {
 
@@ -82,7 +83,7 @@ k_list_chunks(const __grid_constant__ MeshArgs a, const __grid_constant__ Tables
   using S = ListSlot<N>;
   constexpr int T = list_threads<N>(kBig);
   // the dependent launch may start once every CTA is past this point
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using M = ListSmem<N, GM>;
   ChunkSmem<N, VOX_LAYOUT_VERTEX> s;
@@ -460,7 +461,7 @@ k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
     }
   }
   // the generation launch has completed too before this one does
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
 }
 
 // ------------------------------------------------------------------------------------
