@@ -56,9 +56,13 @@ struct RasterArgs {
 // Renders the faces into rgba (width x height x 4 bytes); keys: width x height u64.
 cudaError_t launch_raster(const RasterArgs& a, unsigned long long* keys, uint8_t* rgba,
                           cudaStream_t st);
+struct BatchCtl;
+// The draw list of n chunks; state: look-back words of draw_list_tiles(n) tiles.
+int draw_list_tiles(int n);
 cudaError_t launch_draw_list(const Planes& planes, const void* coords,
                              const unsigned long long* offs, int n, int extent, int instanced,
-                             DrawRecord* out, uint32_t* count, unsigned* err, cudaStream_t st);
+                             DrawRecord* out, uint32_t* count, BatchCtl* ctl, unsigned long long* state,
+                             int spin_limit, cudaStream_t st);
 
 // Neighbour lookup of the staged-halo path (vox_halo.cu): a hash map of the batch's
 // coordinates (cap_mask + 1 slots, a power of two at least twice n), then per chunk and
@@ -83,7 +87,6 @@ struct HaloLookup {
 };
 cudaError_t launch_halo_lookup(const HaloLookup& h, cudaStream_t st);
 
-struct BatchCtl;
 // One look-back for chunk 1 of a batch whose chunk 0 never publishes: the wait must give
 // up after spin_limit polls and latch the timeout bit in ctl (the bounded-wait self-test).
 cudaError_t launch_lookback_probe(unsigned long long* state2, BatchCtl* ctl, int spin_limit,

@@ -4,6 +4,8 @@
 // touches anything that earlier work of the stream writes or reads: the wait ends when all of
 // that work is complete and visible. What is saved is the launch latency between dependent
 // kernels, about a microsecond each; a kernel that follows one without a trigger starts as usual.
+// A kernel whose dependent reads anything before its own pdl_wait triggers after pdl_wait itself
+// (or is launched without this attribute), so that everything ahead of both has ended by then.
 #pragma once
 
 #include <cstring>

@@ -82,23 +82,25 @@ k_list_chunks(const __grid_constant__ MeshArgs a, const __grid_constant__ Tables
   using P = SmemPlan<N, VOX_LAYOUT_VERTEX>;
   using S = ListSlot<N>;
   constexpr int T = list_threads<N>(kBig);
-  // the dependent launch may start once every CTA is past this point
-  pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using M = ListSmem<N, GM>;
   ChunkSmem<N, VOX_LAYOUT_VERTEX> s;
   M::carve(s, smem_raw);
   unsigned char* const lists = M::lists(smem_raw);
   const int i = blockIdx.x, t = threadIdx.x;
+  constexpr bool kHashed = GM == GM_HEIGHT && N <= 32;
+  if (GM != GM_OCC) {  // the context's tables are older than any launch of the stream
+    load_tables<N, VOX_LAYOUT_VERTEX>(s, &tab);
+    if (kHashed) load_grad2<T>(s, reinterpret_cast<float2*>(lists), a.grad2);
+  }
+  pdl_wait();
+  // Only now: k_emit_lists does not wait for earlier work itself, so it must not start, and read
+  // the epoch, before the launches ahead of this one have ended.
+  pdl_trigger();
   unsigned epoch = 0;
   if (t == 0) epoch = ld_relaxed_u32(&a.ctl->epoch);
   const vox_chunk_coord c = a.coords[i];
-  constexpr bool kHashed = GM == GM_HEIGHT && N <= 32;
-  if (GM != GM_OCC) {
-    load_tables<N, VOX_LAYOUT_VERTEX>(s, &tab);
-    if (kHashed) load_grad2<T>(s, reinterpret_cast<float2*>(lists), a.grad2);
-    __syncthreads();
-  }
+  if (GM != GM_OCC) __syncthreads();
   prepare_chunk<N, GM, VOX_LAYOUT_VERTEX, T, kHashed>(s, a, i, c);
   s.stage = lists + M::kLists;
   const uint32_t total = count_and_scan<N, VOX_LAYOUT_VERTEX, T>(s);
@@ -362,6 +364,7 @@ k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
   __shared__ uint32_t s_lists[kEmitThreads / 32 * kWarpFaces];
   __shared__ unsigned long long s_base0;
   __shared__ unsigned s_epoch;
+  pdl_trigger();  // (a launch behind this one waits for its end before it touches anything)
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   Store store;
   store.init(s_table, s_bufs, tab);
@@ -499,6 +502,8 @@ k_mesh_single(const __grid_constant__ MeshArgs a, const __grid_constant__ Tables
   const int t = threadIdx.x, lane = t & 31;
   FaceStore<LAYOUT> store;
   store.init(s_table, smem_raw + M::kBytes + T / 32 * kWarpFaces * 4, tab);
+  pdl_trigger();
+  pdl_wait();
   unsigned use = 0;
   for (int d = 0; d < 6; ++d)
     if (a.occ_nbr[d] && (d < 4 || a.full6)) use |= 1u << d;
