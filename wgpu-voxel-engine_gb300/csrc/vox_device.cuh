@@ -140,8 +140,10 @@ struct SmemPlan {
   // heightmap corner tables: per-octave header, then the gradient coefficients (gx, gy)
   static constexpr int kHHdr = align16((4 * kOctGroup + 1) * 4);
   static constexpr int kHeight = kColK + kAxis + kHHdr + dens_max_corners<N>() * 8;
-  static constexpr int kGenScratch =
-      kHeight > dens_scratch_bytes<N>() ? kHeight : dens_scratch_bytes<N>();
+  // hashed heightmap columns (up to 32^3): the hashed gradients, then the lattice data
+  static constexpr int kHashed = N > 32 ? 0 : kGrad2 * 8 + 2 * kOctGroup * (N + 2) * 16;
+  static constexpr int kScratch0 = kHeight > kHashed ? kHeight : kHashed;
+  static constexpr int kGenScratch = kScratch0 > dens_scratch_bytes<N>() ? kScratch0 : dens_scratch_bytes<N>();
   // staging area: stage_faces / kWarpBatch buffers per warp when staging (stage_faces
   // 32 or 64), else only the generation scratch
   __host__ __device__ static int stage_bytes(int threads, int stage_faces) {
@@ -234,6 +236,18 @@ __device__ __forceinline__ float d_noise2_axes(const uint8_t* p, const float4* g
   const float l0 = d_lerp(ax.u, d_grad2(gt, p[p[A]], x, y), d_grad2(gt, p[p[B]], x1, y));
   const float l1 =
       d_lerp(ax.u, d_grad2(gt, p[p[A + 1]], x, y1), d_grad2(gt, p[p[B + 1]], x1, y1));
+  return d_lerp(az.v, l0, l1);
+}
+
+// The same with the gradients of the hashed corners in a table (entry A: gradient of p[p[A]]).
+__device__ __forceinline__ float d_noise2_hashed(const float2* grad2, const AxisX& ax, const AxisZ& az) {
+  const float2* A = grad2 + ax.px + az.y;
+  const float2* B = grad2 + ax.px1 + az.y;
+  const float2 g00 = A[0], g01 = A[1], g10 = B[0], g11 = B[1];
+  const float x = ax.fr, y = az.fr;
+  const float x1 = x - 1.0f, y1 = y - 1.0f;
+  const float l0 = d_lerp(ax.u, g00.x * x + g00.y * y, g10.x * x1 + g10.y * y);
+  const float l1 = d_lerp(ax.u, g01.x * x + g01.y * y1, g11.x * x1 + g11.y * y1);
   return d_lerp(az.v, l0, l1);
 }
 
@@ -345,7 +359,10 @@ struct ChunkSmem {
   int* hhdr;        // heightmap corner tables: per octave base, corners along z, first x, first z;
                     // [4 * kOctGroup] = corner count, or -1 when the tables are not used
   float2* hcorner;  // heightmap corner gradient coefficients (gx, gy)
-  const float2* grad2;  // gradients of the hashed corners (512), or unused
+  // heightmap columns up to 32^3 (ColumnHash): lattice data per octave and coordinate (x, then z), and
+  // the gradients of the hashed corners; unused otherwise
+  AxisX* hax;
+  const float2* grad2;
 
   __device__ void carve(unsigned char* base) { carve(base, SmemPlan<N, LAYOUT>::list_bytes(blockDim.x)); }
   __device__ void carve(unsigned char* base, int list_bytes) {
@@ -389,12 +406,14 @@ __device__ __forceinline__ void load_tables(ChunkSmem<N, LAYOUT>& s, const Table
   for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
 }
 
-// The hashed gradient table (MeshArgs::grad2, kGrad2 entries) into shared memory at dst.
+// The hashed gradient table (MeshArgs::grad2, kGrad2 entries) into shared memory at dst, with the
+// lattice data's place behind it.
 template <int T, int N, int LAYOUT>
-__device__ __forceinline__ void load_grad2(ChunkSmem<N, LAYOUT>& s, float2* dst, const float2* src) {
+__device__ __forceinline__ void load_grad2(ChunkSmem<N, LAYOUT>& s, unsigned char* dst, const float2* src) {
   const float4* from = reinterpret_cast<const float4*>(src);
   for (int i = threadIdx.x; i < kGrad2 / 2; i += T) reinterpret_cast<float4*>(dst)[i] = __ldg(from + i);
-  s.grad2 = dst;
+  s.grad2 = reinterpret_cast<const float2*>(dst);
+  s.hax = reinterpret_cast<AxisX*>(dst + kGrad2 * 8);
 }
 
 // Write one ballot word for the element run [e0, e0 + 32) of a row-major bit array
@@ -434,13 +453,26 @@ __device__ __forceinline__ void halo_coord(int h, int a, int b, int& x, int& y, 
   }
 }
 
+// k = ceil(base + amp * fbm) - oy clamped to [-1, N + 1] (-1 for NaN): voxel (x, y, z) of a
+// column is solid iff y < k.
+template <int N>
+__device__ __forceinline__ int threshold(const GenDev& g, float fbm, int oy) {
+  const float h = g.base + g.amp * fbm;
+  const float cl = ceilf(h);
+  long long kk = (long long)cl - (long long)oy;
+  if (!(cl == cl)) kk = -1;
+  return (int)(kk < -1 ? -1 : (kk > N + 1 ? N + 1 : kk));
+}
+
+// How heightmap columns up to 32^3 get their lattice data. kHashAll: also from shared tables.
+enum ColumnHash : int { kHashNone = 0, kHashGrad = 1, kHashAll = 2 };
+
 // Threshold of one column (local x, z in -1..N), computed by the calling lane alone: the
-// fBm of the per-column path (d_noise2_axes with the lattice data of this column), then
-// k = ceil(base + amp * fbm) - oy clamped to [-1, N + 1] (-1 for NaN), so that voxel
-// (x, y, z) is solid iff y < k. The same operations, in the same order, as the shared-table
-// path below and as the oracle. With kHashed, s.grad2 holds the gradients of the hashed corners
-// (entry A = gradient of p[p[A]]), so a corner is one load instead of a chain of three.
-template <int N, bool kHashed = false, int LAYOUT>
+// fBm of the per-column path (d_noise2_axes with the lattice data of this column). The same
+// operations, in the same order, as the shared-table paths below and as the oracle. With
+// kHash, s.grad2 holds the gradients of the hashed corners (entry A: the gradient of p[p[A]]),
+// so a corner is one load instead of a chain of three.
+template <int N, int kHash = kHashNone, int LAYOUT>
 __device__ __forceinline__ int column_k(const ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox,
                                         int oy, int oz, int x, int z) {
   const uint8_t* p = s.tab->perm;
@@ -460,25 +492,64 @@ __device__ __forceinline__ int column_k(const ChunkSmem<N, LAYOUT>& s, const Gen
     az.fr = cz - flz;
     az.v = d_fade(az.fr);
     az.pad = 0;
-    if (kHashed) {
-      const float2* A = s.grad2 + ax.px + az.y;
-      const float2* B = s.grad2 + ax.px1 + az.y;
-      const float2 g00 = A[0], g01 = A[1], g10 = B[0], g11 = B[1];
-      const float x0 = ax.fr, y0 = az.fr, x1 = x0 - 1.0f, y1 = y0 - 1.0f;
-      const float l0 = d_lerp(ax.u, g00.x * x0 + g00.y * y0, g10.x * x1 + g10.y * y0);
-      const float l1 = d_lerp(ax.u, g01.x * x0 + g01.y * y1, g11.x * x1 + g11.y * y1);
-      sum = sum + amp * d_lerp(az.v, l0, l1);
-    } else {
-      sum = sum + amp * d_noise2_axes(p, gt, ax, az);
-    }
+    sum = sum + amp * (kHash != kHashNone ? d_noise2_hashed(s.grad2, ax, az) : d_noise2_axes(p, gt, ax, az));
     f = f * g.lac;
     amp = amp * g.gain;
   }
-  const float h = g.base + g.amp * sum;
-  const float cl = ceilf(h);
-  long long kk = (long long)cl - (long long)oy;
-  if (!(cl == cl)) kk = -1;
-  return (int)(kk < -1 ? -1 : (kk > N + 1 ? N + 1 : kk));
+  return threshold<N>(g, sum, oy);
+}
+
+// The same from the lattice data of the chunk's x and z coordinates (hashed_axes) too: a column
+// and octave is two axis entries and four gradients, without the two floors and fades.
+template <int N, int LAYOUT>
+__device__ __forceinline__ int column_k_hashed(const ChunkSmem<N, LAYOUT>& s, const GenDev& g, int oy,
+                                               int x, int z) {
+  constexpr int side = N + 2;
+  const AxisX* pax = s.hax + x + 1;
+  const AxisZ* paz = reinterpret_cast<const AxisZ*>(s.hax + kOctGroup * side) + z + 1;
+  float amp = 1.0f, sum = 0.0f;
+  for (int o = 0; o < g.octaves; ++o) {
+    const AxisX ax = pax[o * side];
+    const AxisZ az = paz[o * side];
+    sum = sum + amp * d_noise2_hashed(s.grad2, ax, az);
+    amp = amp * g.gain;
+  }
+  return threshold<N>(g, sum, oy);
+}
+
+// The lattice data that column_k_hashed reads, for every x and z coordinate and up to kOctGroup
+// octaves (all threads; ends with a barrier).
+template <int N, int T, int LAYOUT>
+__device__ __forceinline__ void hashed_axes(const ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, int oz) {
+  constexpr int side = N + 2;
+  const uint8_t* p = s.tab->perm;
+  AxisX* pax = s.hax;
+  AxisZ* paz = reinterpret_cast<AxisZ*>(s.hax + kOctGroup * side);
+  for (int i = threadIdx.x; i < 2 * side * g.octaves; i += T) {
+    const int o = i / (2 * side), r = i % (2 * side), k = r % side - 1;
+    float fo = g.freq;
+    for (int q = 0; q < o; ++q) fo = fo * g.lac;
+    const float c = (float)((r < side ? ox : oz) + k) * fo;
+    const float fl = floorf(c);
+    const int L = (int)fl & 255;
+    const float fr = c - fl;
+    if (r < side) {
+      AxisX v;
+      v.px = p[L];
+      v.px1 = p[L + 1];
+      v.fr = fr;
+      v.u = d_fade(fr);
+      pax[o * side + k + 1] = v;
+    } else {
+      AxisZ v;
+      v.y = L;
+      v.fr = fr;
+      v.v = d_fade(fr);
+      v.pad = 0;
+      paz[o * side + k + 1] = v;
+    }
+  }
+  __syncthreads();
 }
 
 // Heightmap chunk. Column thresholds colk[(z+1)*(N+2) + (x+1)] = ceil(h(x, z)) - oy,
@@ -487,18 +558,23 @@ __device__ __forceinline__ int column_k(const ChunkSmem<N, LAYOUT>& s, const Gen
 // octave: the lattice data of every x and z coordinate are computed once per octave,
 // each thread accumulating its own columns in registers.
 //
-// Two ways to the thresholds. The direct path (chunks up to 32^3): every lane of the row
-// phase below computes the threshold of its own column itself, with no shared lattice data,
-// so generation needs no CTA barrier before the row ballots. The shared-table path (larger
-// chunks): the lattice data and corner tables are built once per octave in shared memory,
+// Three ways to the thresholds. Up to 32^3 every lane of the row phase below computes the
+// threshold of its own column, with no shared lattice data, so that generation needs no CTA
+// barrier before the row ballots; the list kernel hashes corners by table (kHashGrad), and
+// k_generate, which has no latency to hide behind a count, also reads the coordinates' lattice
+// data from a table (kHashAll: cubes of 1500 terrain chunks of 32^3 37.0 -> 34.9 us; in the list
+// kernel it gained nothing at 16^3 and cost 5 % with one octave). The shared-table path (larger chunks): the lattice data and corner tables are built once per octave in shared memory,
 // every thread accumulates its columns, and the thresholds go through s.colk.
-template <int N, int LAYOUT, int T, bool kHashed>
+template <int N, int LAYOUT, int T, int kHash>
 __device__ void gen_heightmap(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, int oy, int oz,
                               unsigned halo_mask, bool with_halo) {
   using RowT = typename Shape<N>::RowT;
   constexpr int side = N + 2;
   constexpr bool direct = N <= 32;
   const int t = threadIdx.x;
+  // the lattice data are worth their barrier from three octaves on
+  const bool axes = kHash == kHashAll && g.octaves >= 3 && g.octaves <= kOctGroup;
+  if (axes) hashed_axes<N, T>(s, g, ox, oz);
   if (!direct) {
     constexpr int CPT = (side * side + T - 1) / T;
     const uint8_t* p = s.tab->perm;
@@ -640,11 +716,7 @@ __device__ void gen_heightmap(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, 
     for (int c = 0; c < CPT; ++c) {
       const int j = t + c * T;
       if (j < side * side) {
-        const float h = g.base + g.amp * acc[c];
-        const float cl = ceilf(h);
-        long long kk = (long long)cl - (long long)oy;
-        if (!(cl == cl)) kk = -1;
-        s.colk[j] = (int)(kk < -1 ? -1 : (kk > N + 1 ? N + 1 : kk));
+        s.colk[j] = threshold<N>(g, acc[c], oy);
       }
     }
     __syncthreads();
@@ -685,7 +757,9 @@ __device__ void gen_heightmap(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, 
       }
       int k = -1;
       if (used) {
-        k = direct ? column_k<N, kHashed>(s, g, ox, oy, oz, x, z) : s.colk[(z + 1) * side + x + 1];
+        if (!direct) k = s.colk[(z + 1) * side + x + 1];
+        else if (axes) k = column_k_hashed<N>(s, g, oy, x, z);
+        else k = column_k<N, kHash>(s, g, ox, oy, oz, x, z);
       }
       const int kmin = __reduce_min_sync(0xffffffffu, k), kmax = __reduce_max_sync(0xffffffffu, k);
       uint32_t keep[YP];
@@ -1247,14 +1321,14 @@ __device__ bool gen_density(ChunkSmem<N, LAYOUT>& s, const GenDev& g, int ox, in
 
 // Fills s.occ (own rows) and, for every set bit of `halo_mask`, the halo rows; the other
 // halo rows are zero (a neighbour that is not loaded counts as air, chunk.rs:102-107).
-// kHashed: s.grad2 holds the hashed gradients of the heightmap columns (see column_k).
-template <int N, int GM, int LAYOUT, int T, bool kHashed = false>
+// kHash: where heightmap columns get their lattice data (see column_k).
+template <int N, int GM, int LAYOUT, int T, int kHash = kHashNone>
 __device__ void gen_chunk(ChunkSmem<N, LAYOUT>& s, const GenDev& g, vox_chunk_coord c,
                           long long chunk_index, unsigned halo_mask, bool with_halo) {
   using RowT = typename Shape<N>::RowT;
   const int ox = c.x * N, oy = c.y * N, oz = c.z * N;
   if (GM == GM_HEIGHT) {
-    gen_heightmap<N, LAYOUT, T, kHashed>(s, g, ox, oy, oz, halo_mask, with_halo);
+    gen_heightmap<N, LAYOUT, T, kHash>(s, g, ox, oy, oz, halo_mask, with_halo);
     return;
   }
   if (GM == GM_DENSITY) {
@@ -2169,7 +2243,7 @@ __host__ __device__ constexpr int fused_min_ctas() {
 // meshing of resident occupancy (GM == GM_OCC). One chunk per CTA iteration; T threads.
 // Occupancy and halo rows of chunk i in shared memory: loaded from the slot pool
 // (GM_OCC) or generated from the noise field.
-template <int N, int GM, int LAYOUT, int T, bool kHashed = false>
+template <int N, int GM, int LAYOUT, int T, int kHash = kHashNone>
 __device__ __forceinline__ void prepare_chunk(ChunkSmem<N, LAYOUT>& s, const MeshArgs& a, int i,
                                               vox_chunk_coord c) {
   if (GM == GM_OCC) {
@@ -2196,7 +2270,7 @@ __device__ __forceinline__ void prepare_chunk(ChunkSmem<N, LAYOUT>& s, const Mes
     unsigned m = a.nbr_mask ? a.nbr_mask[i] : 0u;
     if (GM == GM_BERNOULLI) m = 0u;
     if (!a.full6) m &= 0xFu;
-    gen_chunk<N, GM, LAYOUT, T, kHashed>(s, a.gen, c, a.index_base + i, m, true);
+    gen_chunk<N, GM, LAYOUT, T, kHash>(s, a.gen, c, a.index_base + i, m, true);
   }
 }
 
@@ -2740,9 +2814,10 @@ k_generate(MeshArgs a, uint32_t* occ_out) {
   }
   load_tables<N, VOX_LAYOUT_VERTEX>(s, a.tables);
   constexpr bool kHashed = GM == GM_HEIGHT && N <= 32;
-  if (kHashed) load_grad2<T>(s, reinterpret_cast<float2*>(s.stage), a.grad2);
+  if (kHashed) load_grad2<T>(s, s.stage, a.grad2);
   __syncthreads();
-  gen_chunk<N, GM, VOX_LAYOUT_VERTEX, T, kHashed>(s, a.gen, a.coords[i], a.index_base + i, 0u, false);
+  gen_chunk<N, GM, VOX_LAYOUT_VERTEX, T, kHashed ? kHashAll : kHashNone>(s, a.gen, a.coords[i],
+                                                                         a.index_base + i, 0u, false);
   const uint32_t* src = reinterpret_cast<const uint32_t*>(s.occ);
   uint32_t* dst = occ_out + (size_t)slot * words;
   for (int q = threadIdx.x; q < words; q += blockDim.x) dst[q] = src[q];

@@ -91,7 +91,7 @@ k_list_chunks(const __grid_constant__ MeshArgs a, const __grid_constant__ Tables
   constexpr bool kHashed = GM == GM_HEIGHT && N <= 32;
   if (GM != GM_OCC) {  // the context's tables are older than any launch of the stream
     load_tables<N, VOX_LAYOUT_VERTEX>(s, &tab);
-    if (kHashed) load_grad2<T>(s, reinterpret_cast<float2*>(lists), a.grad2);
+    if (kHashed) load_grad2<T>(s, lists, a.grad2);
   }
   pdl_wait();
   // Only now: k_emit_lists does not wait for earlier work itself, so it must not start, and read
@@ -101,7 +101,7 @@ k_list_chunks(const __grid_constant__ MeshArgs a, const __grid_constant__ Tables
   if (t == 0) epoch = ld_relaxed_u32(&a.ctl->epoch);
   const vox_chunk_coord c = a.coords[i];
   if (GM != GM_OCC) __syncthreads();
-  prepare_chunk<N, GM, VOX_LAYOUT_VERTEX, T, kHashed>(s, a, i, c);
+  prepare_chunk<N, GM, VOX_LAYOUT_VERTEX, T, kHashed ? kHashGrad : kHashNone>(s, a, i, c);
   s.stage = lists + M::kLists;
   const uint32_t total = count_and_scan<N, VOX_LAYOUT_VERTEX, T>(s);
   unsigned char* dst = reinterpret_cast<unsigned char*>(a.scratch) + (unsigned long long)i * S::kBytes;
