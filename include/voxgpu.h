@@ -237,9 +237,10 @@ int vox_gen_mesh_host(vox_ctx* ctx, const vox_chunk_coord* h_coords, const uint8
 
 /* ---- Tuning ------------------------------------------------------------------------------ */
 
-/* Launch shape of the meshing kernels. threads, stage_faces and ctas_per_sm shape every launch
- * but those of the overlap schedule into device memory, except for VOX_GEN_BERNOULLI, whose two
- * launches (face lists, then records) have shapes of their own. */
+/* Launch shape of the meshing kernels. With the shape of an untuned context (vox_ctx_get_tuning
+ * after vox_ctx_create) the overlap schedule into device memory is two launches (face lists, then
+ * records) with shapes of their own, where these are the faster way; every other shape is that of
+ * one persistent launch. */
 typedef struct vox_tuning {
   int32_t threads;     /* CTA size; each chunk size has two (8: 32/64, 16: 128/256,
                           32: 256/512, 64: 512/1024) */
@@ -275,7 +276,7 @@ typedef struct vox_tuning {
  * OVERLAP: the phases of PHASED without the grid barrier: each chunk's total is published
  *   as soon as it is counted, and emission takes a chunk's offset from a decoupled
  *   look-back over the published totals, so emission overlaps the end of generation. Into
- *   device memory (except VOX_GEN_BERNOULLI) the phases are two launches, of which the second
+ *   device memory and with the default shape the phases are two launches, of which the second
  *   starts while the first still runs. */
 enum { VOX_SCHEDULE_LOOKBACK = 0, VOX_SCHEDULE_PHASED = 1, VOX_SCHEDULE_OVERLAP = 2 };
 

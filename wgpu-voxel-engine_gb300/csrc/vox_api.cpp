@@ -273,15 +273,33 @@ int apply_tuning(vox_ctx* ctx, int topt, int stage_faces, int ctas_per_sm, int s
   return VOX_OK;
 }
 
-// Whether a launch goes through the face lists (vox_lists.cuh): the overlap schedule with
-// outputs in device memory, unless the voxels are random, whose chunks never fit a list.
-bool use_lists(const vox_ctx* ctx, int gm, bool host_out) {
-  return ctx->schedule == VOX_SCHEDULE_OVERLAP && !host_out && gm != GM_BERNOULLI;
+// The launch shape of a context that was not tuned; under the overlap schedule into device
+// memory it stands for the list launches, whose shapes are their own.
+bool default_shape(const vox_ctx* ctx, int topt, int stage_faces, int ctas_per_sm) {
+  return topt == default_topt(ctx->cfg.chunk_size) && stage_faces == kStageSingle && ctas_per_sm == 0;
+}
+
+// Whether a launch of n chunks goes through the face lists (vox_lists.cuh): the overlap schedule
+// with the default shape and outputs in device memory, unless the voxels are random, whose
+// chunks never fit a list. Large batches of small heightmap chunks in the vertex layout stay
+// with the persistent launch: from two rounds of list CTAs on (2432 chunks of 16^3, 9728 of
+// 8^3) emission that overlaps generation from the start is worth more than occupancy. us a
+// batch, lists / one launch: 16^3 2000 chunks 50 / 52, 3000 69 / 71 (128 threads: 66), 4000
+// 93 / 91 (85), 8000 181 / 171 (153); 8^3 4000 38 / 46, 16000 108 / 101. Lists stay ahead for
+// instances (16^3, 8000 chunks 126 / 156), caves (16^3, 4000 chunks 104 / 113) and from 32^3 on
+// (terrain, 4096 chunks 320 / 344).
+bool use_lists(const vox_ctx* ctx, int gm, int n, bool host_out) {
+  if (ctx->schedule != VOX_SCHEDULE_OVERLAP || host_out || gm == GM_BERNOULLI ||
+      !default_shape(ctx, ctx->topt, ctx->stage_faces, ctx->ctas_per_sm))
+    return false;
+  const int N = ctx->cfg.chunk_size;
+  return N > 16 || gm != GM_HEIGHT || ctx->cfg.layout != VOX_LAYOUT_VERTEX ||
+         n <= 2 * ctx->num_sms * (N == 16 ? 8 : 32);
 }
 
 // Scratch of one chunk of a launch.
-size_t slot_bytes(const vox_ctx* ctx, int gm, bool host_out) {
-  return (size_t)(use_lists(ctx, gm, host_out) ? ctx->ks->list_slot_bytes : ctx->ks->spill_bytes);
+size_t slot_bytes(const vox_ctx* ctx, bool lists) {
+  return (size_t)(lists ? ctx->ks->list_slot_bytes : ctx->ks->spill_bytes);
 }
 
 // Per-chunk scratch and face totals for n chunks (grow; never shrink).
@@ -413,8 +431,8 @@ int issue_lists(vox_ctx* ctx, MeshArgs& a, int gm, cudaStream_t stream) {
 
 // Issues one fused batch launch with the context's tuning on `stream`; the scratch of the
 // schedule (a.state, or a.scratch + a.counts) is already in `a`.
-int issue_batch(vox_ctx* ctx, MeshArgs& a, int gm, bool host_out, cudaStream_t stream) {
-  if (use_lists(ctx, gm, host_out)) return issue_lists(ctx, a, gm, stream);
+int issue_batch(vox_ctx* ctx, MeshArgs& a, int gm, bool host_out, bool lists, cudaStream_t stream) {
+  if (lists) return issue_lists(ctx, a, gm, stream);
   const int layout = ctx->cfg.layout;
   const int threads = ctx->ks->threads[ctx->topt];
   const int smem = ctx->ks->smem_total(layout, threads, host_out ? kStageSingle : ctx->stage_faces);
@@ -580,8 +598,15 @@ int batch_launch(vox_ctx* ctx, MeshArgs& a, int gm, bool host_out = false) {
     gm = GM_OCC;
   }
   const int slab = slab_of(ctx, a.n);
+  bool lists = use_lists(ctx, gm, slab, host_out);
   if (ctx->schedule != VOX_SCHEDULE_LOOKBACK) {  // the spill slots of phases A and C
-    if ((st = ensure_scratch(ctx, (size_t)slab, slot_bytes(ctx, gm, host_out))) != VOX_OK) return st;
+    st = ensure_scratch(ctx, (size_t)slab, slot_bytes(ctx, lists));
+    if (st == VOX_ERR_OOM && lists && ctx->ks->list_slot_bytes > ctx->ks->spill_bytes) {
+      cudaGetLastError();  // 64^3 lists take twice the room of the persistent launch's slots
+      lists = false;
+      st = ensure_scratch(ctx, (size_t)slab, slot_bytes(ctx, lists));
+    }
+    if (st != VOX_OK) return st;
     a.scratch = ctx->d_scratch;
     a.counts = ctx->d_counts;
   }
@@ -596,7 +621,7 @@ int batch_launch(vox_ctx* ctx, MeshArgs& a, int gm, bool host_out = false) {
       const int s2 = before_batch_launch(ctx);
       if (s2 != VOX_OK) return s2;
     }
-    return issue_batch(ctx, b, gm, host_out, ctx->stream);
+    return issue_batch(ctx, b, gm, host_out, lists, ctx->stream);
   });
 }
 
@@ -1250,11 +1275,6 @@ int vox_autotune(vox_ctx* ctx, const vox_chunk_coord* d_coords, const uint8_t* d
       for (int s : stages) {
         int full_grid = 0;
         for (int c : ctas) {
-          // the list launches have shapes of their own: one candidate, with the default shape
-          // (which launches that write host memory use)
-          if (p == VOX_SCHEDULE_OVERLAP && ctx->gm != GM_BERNOULLI &&
-              (t != default_topt(ctx->cfg.chunk_size) || s != kStageSingle || c != 0))
-            continue;
           if (apply_tuning(ctx, t, s, c, p, 0, 0) != VOX_OK) continue;
           const int g = p == VOX_SCHEDULE_PHASED    ? ctx->phased_grid[ctx->gm]
                         : p == VOX_SCHEDULE_OVERLAP ? ctx->overlap_grid[ctx->gm]
@@ -1355,9 +1375,15 @@ int vox_graph_capture(vox_ctx* ctx, const vox_chunk_coord* d_coords, const uint8
   a.face_offsets = reinterpret_cast<unsigned long long*>(d_face_offsets);
   const int slab = slab_of(ctx, n);
   g->launches = (n + slab - 1) / slab;
+  bool lists = use_lists(ctx, ctx->halo_staging ? GM_OCC : ctx->gm, slab, false);
   if (g->schedule != VOX_SCHEDULE_LOOKBACK) {
-    const size_t slot = slot_bytes(ctx, ctx->halo_staging ? GM_OCC : ctx->gm, false);
-    if ((e = cudaMalloc(&g->d_scratch, (size_t)slab * slot)) != cudaSuccess ||
+    e = cudaMalloc(&g->d_scratch, (size_t)slab * slot_bytes(ctx, lists));
+    if (e == cudaErrorMemoryAllocation && lists && ctx->ks->list_slot_bytes > ctx->ks->spill_bytes) {
+      cudaGetLastError();
+      lists = false;
+      e = cudaMalloc(&g->d_scratch, (size_t)slab * slot_bytes(ctx, lists));
+    }
+    if (e != cudaSuccess ||
         (e = cudaMalloc(&g->d_counts, (size_t)slab * sizeof(uint32_t))) != cudaSuccess)
       return bail(cuda_fail(ctx, e, "cudaMalloc(graph scratch)"));
     a.scratch = g->d_scratch;
@@ -1385,7 +1411,7 @@ int vox_graph_capture(vox_ctx* ctx, const vox_chunk_coord* d_coords, const uint8
   int gm = ctx->gm;
   if (ctx->halo_staging && (st = halo_prepass(ctx, a, gm, g->halo, cs)) == VOX_OK) gm = GM_OCC;
   if (st == VOX_OK)
-    st = for_each_slab(a, slab, [&](MeshArgs& b) { return issue_batch(ctx, b, gm, false, cs); });
+    st = for_each_slab(a, slab, [&](MeshArgs& b) { return issue_batch(ctx, b, gm, false, lists, cs); });
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(cs, &graph);
   cudaStreamDestroy(cs);

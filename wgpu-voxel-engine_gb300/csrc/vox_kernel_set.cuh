@@ -58,7 +58,7 @@ static KernelSet make_kernel_set() {
   fill_lists<N, GM_DENSITY>(k);
   k.emit[VOX_LAYOUT_VERTEX] = (const void*)k_emit_lists<N, VOX_LAYOUT_VERTEX>;
   k.emit[VOX_LAYOUT_INSTANCED] = (const void*)k_emit_lists<N, VOX_LAYOUT_INSTANCED>;
-  k.emit_threads = kEmitThreads;
+  k.emit_threads = emit_threads<N>();
   k.list_threads[0] = list_threads<N>(0);
   k.list_threads[1] = list_threads<N>(1);
   k.list_slot_bytes = ListSlot<N>::kBytes;

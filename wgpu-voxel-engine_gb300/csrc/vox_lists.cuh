@@ -211,7 +211,12 @@ static __device__ bool chunk_offset(const MeshArgs& a, unsigned epoch, int i, un
 // buffer with a TMA bulk copy waits about a microsecond for the copy to have read it.
 // ------------------------------------------------------------------------------------
 
-constexpr int kEmitThreads = 256;
+// CTA size of the emission grid, 32 warps an SM either way. From 32^3 on small CTAs fill the
+// places that generation CTAs leave one by one (777 cave chunks 39.5 -> 37.8 us; the same at
+// 16^3: 2000 chunks 51.6 -> 54.5 us). With 40 warps an SM (48 registers) the terrain batch took
+// 37.3 instead of 33.5 us, with 24 warps 42.5.
+template <int N>
+__host__ __device__ constexpr int emit_threads() { return N <= 16 ? 256 : 128; }
 
 // Translations of a chunk: local coordinate q_c of byte c of a face code -> world coordinate
 // o_c + q_c as a float, rounded once. Origins below 2^23 - 64 in size take a shorter way with the
@@ -236,13 +241,20 @@ struct Origin {
   }
 };
 
-template <int LAYOUT>
+// kPad: staging and table entries spread over the banks (41.2 -> 39.5 us on the cave chunks of
+// 32^3; at 16^3 the shorter address arithmetic is worth more, 33.4 against 34.0 us).
+template <int LAYOUT, bool kPad>
 struct FaceStore;
 
-template <>
-struct FaceStore<VOX_LAYOUT_VERTEX> {
-  static constexpr int kTableBytes = 6 * 64;         // per direction 12 corner coordinates, face
-  static constexpr int kBufBytes = kWarpBatch * 96;  // a warp's buffer
+template <bool kPad>
+struct FaceStore<VOX_LAYOUT_VERTEX, kPad> {
+  // Per direction 12 corner coordinates and the face; padded 80 bytes apart, so that the six
+  // directions' entries lie in different banks.
+  static constexpr int kEntry = kPad ? 5 : 4;  // 16-byte units
+  static constexpr int kTableBytes = 6 * kEntry * 16;
+  // A warp's buffer: 16-byte unit u at u, or padded at u + u / 24 (a gap behind every four
+  // records), so that the eight lanes that store a unit together hit different banks.
+  static constexpr int kBufBytes = (kWarpBatch * 6 + (kPad ? kWarpBatch / 4 : 0)) * 16;
   const float4* table;
   float4* buf;
   int lane;
@@ -254,7 +266,7 @@ struct FaceStore<VOX_LAYOUT_VERTEX> {
     buf = reinterpret_cast<float4*>(bufs + (threadIdx.x >> 5) * kBufBytes);
     for (int i = threadIdx.x; i < 6 * 13; i += blockDim.x) {
       const int d = i / 13, k = i % 13;
-      reinterpret_cast<float*>(smem)[d * 16 + k] =
+      reinterpret_cast<float*>(smem)[d * kEntry * 4 + k] =
           k < 12 ? (&tab.corner[d][0][0])[k] : __uint_as_float(tab.slot[d]);
     }
   }
@@ -263,11 +275,11 @@ struct FaceStore<VOX_LAYOUT_VERTEX> {
   template <bool kSmall>
   __device__ __forceinline__ void batch(uint32_t q, int nw, uint32_t first, const Origin& org,
                                         unsigned long long g, void* out0, void* out1) const {
-    const float4* C = table + (q >> 24) * 4u;
+    const float4* C = table + (q >> 24) * (unsigned)kEntry;
     const float4 c0 = C[0], c1 = C[1], c2 = C[2];
     const float face = C[3].x;
     const float tx = org.at<kSmall>(q, 0), ty = org.at<kSmall>(q, 1), tz = org.at<kSmall>(q, 2);
-    float4* v = buf + lane * 6;
+    float4* v = buf + lane * 6 + (kPad ? lane >> 2 : 0);
     __syncwarp();  // the last batch has been copied out
     // position, tex coords (0,0) (1,0) (0,1) (1,1) (src/quad.rs:66-87) and face, 6 words a vertex
     v[0] = make_float4(c0.x + tx, c0.y + ty, c0.z + tz, 0.0f);
@@ -281,7 +293,7 @@ struct FaceStore<VOX_LAYOUT_VERTEX> {
     const int units = nw * 6;
 #pragma unroll
     for (int k = 0; k < 6; ++k)
-      if (32 * k + lane < units) o[32 * k] = buf[32 * k + lane];
+      if (32 * k + lane < units) o[32 * k] = buf[32 * k + lane + (kPad ? (32 * k + lane) / 24 : 0)];
     // indices 4 f + {0, 2, 1, 3, 1, 2}: 8-byte pair j of face u / 3
     uint2* x = reinterpret_cast<uint2*>(reinterpret_cast<unsigned char*>(out1) + g * 24ull) + lane;
 #pragma unroll
@@ -293,8 +305,8 @@ struct FaceStore<VOX_LAYOUT_VERTEX> {
   }
 };
 
-template <>
-struct FaceStore<VOX_LAYOUT_INSTANCED> {
+template <bool kPad>
+struct FaceStore<VOX_LAYOUT_INSTANCED, kPad> {
   static constexpr int kTableBytes = 6 * 80;  // per direction the 17 words of a record
   static constexpr int kBufBytes = kWarpBatch * 68;
   const float* table;
@@ -354,11 +366,12 @@ struct FaceStore<VOX_LAYOUT_INSTANCED> {
 };
 
 template <int N, int LAYOUT>
-__global__ void __launch_bounds__(kEmitThreads, 4)
+__global__ void __launch_bounds__(emit_threads<N>(), 1024 / emit_threads<N>())
 k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesDev tab) {
   using S = ListSlot<N>;
   constexpr unsigned kLine = line_faces<LAYOUT>();
-  using Store = FaceStore<LAYOUT>;
+  constexpr int kEmitThreads = emit_threads<N>();
+  using Store = FaceStore<LAYOUT, (N > 16)>;
   __shared__ __align__(16) unsigned char s_table[Store::kTableBytes];
   __shared__ __align__(16) unsigned char s_bufs[kEmitThreads / 32 * Store::kBufBytes];
   __shared__ uint32_t s_lists[kEmitThreads / 32 * kWarpFaces];
@@ -486,7 +499,7 @@ __host__ __device__ constexpr int single_ctas() { return N == 8 ? 1 : (N == 16 ?
 template <int N, int LAYOUT>
 __host__ __device__ constexpr int single_smem() {
   return ListSmem<N, GM_OCC>::kBytes +
-         single_threads<N>() / 32 * (kWarpFaces * 4 + FaceStore<LAYOUT>::kBufBytes);
+         single_threads<N>() / 32 * (kWarpFaces * 4 + FaceStore<LAYOUT, false>::kBufBytes);
 }
 
 template <int N, int LAYOUT>
@@ -495,12 +508,12 @@ k_mesh_single(const __grid_constant__ MeshArgs a, const __grid_constant__ Tables
   using M = ListSmem<N, GM_OCC>;
   constexpr int T = single_threads<N>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ __align__(16) unsigned char s_table[FaceStore<LAYOUT>::kTableBytes];
+  __shared__ __align__(16) unsigned char s_table[FaceStore<LAYOUT, false>::kTableBytes];
   ChunkSmem<N, VOX_LAYOUT_VERTEX> s;
   M::carve(s, smem_raw);
   s.lists = reinterpret_cast<uint32_t*>(smem_raw + M::kBytes);
   const int t = threadIdx.x, lane = t & 31;
-  FaceStore<LAYOUT> store;
+  FaceStore<LAYOUT, false> store;
   store.init(s_table, smem_raw + M::kBytes + T / 32 * kWarpFaces * 4, tab);
   pdl_trigger();
   pdl_wait();

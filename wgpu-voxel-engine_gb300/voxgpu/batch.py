@@ -9,7 +9,8 @@ memory comes from torch (plumbing only); every launch goes through the C ABI.
 """
 from __future__ import annotations
 
-from . import GEN_BERNOULLI, SCHEDULE_OVERLAP, VOX_OK, VOX_ERR_CAPACITY, VoxError
+from . import (GEN_BERNOULLI, GEN_HEIGHTMAP, LAYOUT_VERTEX, SCHEDULE_OVERLAP, VOX_OK,
+               VOX_ERR_CAPACITY, VoxError)
 
 
 class BatchRun:
@@ -58,13 +59,26 @@ class BatchRun:
             # staged halos: coordinate map (with the identity slots), neighbour lookup,
             # generation of the batch and (with neighbour masks) of the halo planes outside it
             self.launches_per_step += 3 + (1 if masks is not None else 0)
-        # the overlap schedule's batch launch is two kernels: face lists, then records (random
-        # voxels, unless they are staged in a pool: one kernel)
-        two = t.schedule == SCHEDULE_OVERLAP and (ctx.cfg.gen.kind != GEN_BERNOULLI or t.halo_staging)
-        self.kernels_per_step = self.launches_per_step + ((n + slab - 1) // slab if two else 0)
+        self.kernels_per_step = self.launches_per_step + (
+            (n + slab - 1) // slab if self._two_kernels(t, slab) else 0)
         self.graph = (ctx.capture_graph(self.d_coords, self.d_mask, n, self.out0, self.out1,
                                         self.cap, self.offsets, chunk_index_base=index_base)
                       if graph else None)
+
+    def _two_kernels(self, t, slab) -> bool:
+        """Whether a batch launch of `slab` chunks is two kernels (face lists, then records): the
+        library's rule (use_lists in csrc/vox_api.cpp), for counting."""
+        import torch
+        cfg = self.ctx.cfg
+        default = t.threads == {8: 64, 16: 256}.get(cfg.chunk_size, 512) and t.stage_faces == 32
+        if t.schedule != SCHEDULE_OVERLAP or not default or t.ctas_per_sm != 0:
+            return False
+        if t.halo_staging:
+            return True
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        return cfg.gen.kind != GEN_BERNOULLI and (
+            cfg.chunk_size > 16 or cfg.gen.kind != GEN_HEIGHTMAP or cfg.layout != LAYOUT_VERTEX
+            or slab <= 2 * sms * (8 if cfg.chunk_size == 16 else 32))
 
     def launch(self):
         """One pass over the batch (asynchronous on the context's stream)."""
