@@ -194,9 +194,15 @@ __device__ __forceinline__ f2_t f2_mul(f2_t a, f2_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-// d_lerp on both halves
-__device__ __forceinline__ f2_t f2_lerp(f2_t t, f2_t a, f2_t b) {
-  return f2_add(a, f2_mul(t, f2_sub(b, a)));
+// d_lerp on both halves. nz holds {-0, -0} that the compiler does not know: a mul.f32x2 whose
+// product only an add.f32x2 takes can come out as one fused operation, in spite of -fmad=false
+// and .rn, whose single rounding flips about one voxel in 10^10 (a product that the
+// gradients' coefficients 0 and +-1 make exact is the same either way). As an fma with -0 the
+// product is rounded by itself, sign of zero included.
+__device__ __forceinline__ f2_t f2_lerp(f2_t t, f2_t a, f2_t b, f2_t nz) {
+  f2_t m;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(m) : "l"(t), "l"(f2_sub(b, a)), "l"(nz));
+  return f2_add(a, m);
 }
 // Gradient dot products from the coefficient table (gx, gy, gz) of hash & 15.
 __device__ __forceinline__ float d_grad3(const float4* gt, int h, float x, float y, float z) {
@@ -1034,6 +1040,7 @@ __device__ __forceinline__ uint32_t dens_block_z(const ChunkSmem<N, LAYOUT>& s, 
   const ulonglong2* axes = reinterpret_cast<const ulonglong2*>(s.stage + P::kAxes);
   const ulonglong2* pair_xy = reinterpret_cast<const ulonglong2*>(s.stage + P::kPairXY);
   const f2_t* pair_z = reinterpret_cast<const f2_t*>(s.stage + P::kPairZ);
+  const f2_t nz = f2_pack(g.neg_zero, g.neg_zero);
   float sum[kDensB];
 #pragma unroll
   for (int i = 0; i < kDensB; ++i) sum[i] = 0.0f;
@@ -1071,10 +1078,10 @@ __device__ __forceinline__ uint32_t dens_block_z(const ChunkSmem<N, LAYOUT>& s, 
       const f2_t d10 = f2_add(q10, f2_mul(z10, zr.x));
       const f2_t d01 = f2_add(q01, f2_mul(z01, zr.x));
       const f2_t d11 = f2_add(q11, f2_mul(z11, zr.x));
-      const f2_t l0 = f2_lerp(uu, d00, d10);  // {l00, l01}
-      const f2_t l1 = f2_lerp(uu, d01, d11);  // {l10, l11}
+      const f2_t l0 = f2_lerp(uu, d00, d10, nz);  // {l00, l01}
+      const f2_t l1 = f2_lerp(uu, d01, d11, nz);  // {l10, l11}
       float m0, m1;
-      f2_unpack(f2_lerp(vv, l0, l1), m0, m1);
+      f2_unpack(f2_lerp(vv, l0, l1, nz), m0, m1);
       sum[i] = sum[i] + amp * d_lerp(__uint_as_float((unsigned)zr.y), m0, m1);
     }
     amp = amp * g.gain;
@@ -1103,6 +1110,7 @@ __device__ __forceinline__ uint32_t dens_block_y(const ChunkSmem<N, LAYOUT>& s, 
   const DensAxis* axes = reinterpret_cast<const DensAxis*>(s.stage + P::kAxes);
   const ulonglong2* pair_xy = reinterpret_cast<const ulonglong2*>(s.stage + P::kPairXY);
   const f2_t* pair_z = reinterpret_cast<const f2_t*>(s.stage + P::kPairZ);
+  const f2_t nz = f2_pack(g.neg_zero, g.neg_zero);
   float sum[kDensY];
 #pragma unroll
   for (int i = 0; i < kDensY; ++i) sum[i] = 0.0f;
@@ -1140,10 +1148,10 @@ __device__ __forceinline__ uint32_t dens_block_y(const ChunkSmem<N, LAYOUT>& s, 
       const f2_t d10 = f2_add(f2_add(px10, f2_mul(gy10, ya2)), pz10);
       const f2_t d01 = f2_add(f2_add(px01, f2_mul(gy01, yb2)), pz01);
       const f2_t d11 = f2_add(f2_add(px11, f2_mul(gy11, yb2)), pz11);
-      const f2_t l0 = f2_lerp(uu, d00, d10);  // {l00, l01}
-      const f2_t l1 = f2_lerp(uu, d01, d11);  // {l10, l11}
+      const f2_t l0 = f2_lerp(uu, d00, d10, nz);  // {l00, l01}
+      const f2_t l1 = f2_lerp(uu, d01, d11, nz);  // {l10, l11}
       float m0, m1;
-      f2_unpack(f2_lerp(f2_pack(ay.fade, ay.fade), l0, l1), m0, m1);
+      f2_unpack(f2_lerp(f2_pack(ay.fade, ay.fade), l0, l1, nz), m0, m1);
       sum[i] = sum[i] + amp * d_lerp(az.fade, m0, m1);
     }
     amp = amp * g.gain;

@@ -26,6 +26,7 @@ struct GenDev {
   unsigned long long seed;
   float freq, lac, gain, amp, base, y_ref, y_scale;
   int solid_below_zero;
+  float neg_zero = -0.0f;  // see f2_lerp
 };
 
 // Per-context constant tables, computed on the host once (see vox_tables.cpp).
