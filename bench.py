@@ -56,6 +56,12 @@ L2_FLUSH_BYTES = 256 << 20
 # written by one launch; for stress the capture ran on 48 chunks and the figure is scaled
 # to the launch's chunk count (DRAM bytes grow with the faces written).
 NCU = {
+    ("k_list_chunks + k_emit_lists", "heightmap"): {
+        "traffic": 9170000, "warp_instructions": 13748599, "chunks": 1024, "per_step": True,
+        "summary": "profiles/face_lists.md"},
+    ("k_list_chunks + k_emit_lists", "density"): {
+        "traffic": 617600000, "warp_instructions": 143786463, "chunks": 4096, "per_step": True,
+        "summary": "profiles/face_lists.md"},
     ("k_mesh_batch_overlap", "heightmap"): {
         "traffic": 7112704, "warp_instructions": 18389229, "chunks": 1024,
         "summary": "profiles/k_mesh_batch_overlap_heightmap.md"},
@@ -227,15 +233,9 @@ ISSUE_PEAK = 152 * 4 * 2.07e9
 # (7 each), corner gradients (2-D: 2 mul + 1 add; 3-D: 3 mul + 2 add), lerps (3 each),
 # the coordinate scaling and the fBm update (sum, amp, f).
 NOISE_OPS = {2: 2 + 2 + 14 + 2 + 4 * 3 + 3 * 3 + 2 + 4, 3: 3 + 3 + 21 + 3 + 8 * 5 + 7 * 3 + 3 + 4}
-# FP32 lane operations the kernels execute per sample-octave. The 2-D heightmap path
-# evaluates the whole formula per column. The 3-D lattice-table paths compute the per-axis
-# parts (floors, fractions, fades) once per coordinate: per sample they execute the corner
-# dot products, the lerps and the fBm sum (8 x 5 + 7 x 3 + 3 = 64). The 32^3 lane = z path
-# holds g.y * y and g.z * z per corner record and evaluates corner pairs as f32x2 (two lanes
-# per instruction): 4 dot pairs (1 mul + 2 adds), 2 x-lerp pairs and 1 y-lerp pair
-# (3 each) = 21 x 2, the z lerp and the sum (5), and the record products (8 pairs, at
-# least once per 8 samples: 2) = 49.
-NOISE_EXEC_OPS = {"2d": NOISE_OPS[2], "3d_table": 64, "3d_lane_z": 49}
+# The 2-D heightmap paths evaluate the whole formula per column. The 3-D density paths decide
+# most samples without evaluating them (bounds of the noise, coarse samples), so their rate in
+# formula operations is no FP32 utilisation and no executed count is reported.
 # FP32 lane rate: 152 SMs x 128 lanes x 2.07 GHz, one operation per lane per cycle (an f32x2
 # instruction is two). Nominal: the measured peaks file has no FP32 figure.
 FP32_OPS_NOMINAL = 152 * 128 * 2.07e9
@@ -243,44 +243,36 @@ FP32_PEAK_SOURCE = ("nominal FP32 lane rate (152 SMs x 128 lanes x 2.07 GHz, FMA
                     "the measured-peaks file has no FP32 figure")
 
 
-def own_noise_ops(cfg):
-    """Executed FP32 lane operations per sample-octave of a chunk's own samples."""
-    if cfg.gen.kind == 0:
-        return NOISE_EXEC_OPS["2d"]
-    return NOISE_EXEC_OPS["3d_lane_z" if cfg.chunk_size == 32 else "3d_table"]
+def noise_rates(kind, total, octaves, seconds):
+    """The noise of `total` samples in `seconds`: the formula's operations per second and, where
+    every sample is evaluated (heightmap columns), their share of the FP32 lane rate."""
+    dim = 2 if kind == 0 else 3
+    formula = total * octaves * NOISE_OPS[dim] / seconds
+    out = {"octaves": octaves, "formula_ops_per_sample_octave": NOISE_OPS[dim],
+           "formula_tops": formula / 1e12}
+    if kind == 0:
+        out |= {"achieved_tops": formula / 1e12, "peak_tops": FP32_OPS_NOMINAL / 1e12,
+                "peak_source": FP32_PEAK_SOURCE, "frac": formula / FP32_OPS_NOMINAL}
+    else:
+        out["samples"] = ("covered, not evaluated: chunks and cells that the noise's bounds and "
+                          "coarse samples decide cost no noise")
+    return out
 
 
 def noise_report(wl, cfg, masks, ms_per_step):
-    """FP32 throughput of the noise in one step: samples x octaves x the lane operations
-    their path executes, against the FP32 lane rate; beside it the rate in formula operations
-    (the per-sample formula's count at the same sample rate)."""
+    """The rate of the noise in one step: samples x octaves in the formula's operations."""
     N = cfg.chunk_size
     g = cfg.gen
     n_chunks = len(masks)
     if g.kind == 0:    # heightmap: 2-D noise per column, (N + 2)^2 - 4 columns with halo
-        samples, dim = (N + 2) ** 2 - 4, 2
-        total = n_chunks * samples
-        ops = total * g.octaves * NOISE_EXEC_OPS["2d"]
+        total = n_chunks * ((N + 2) ** 2 - 4)
     elif g.kind == 1:  # density: 3-D noise per voxel and per halo voxel of a loaded neighbour
-        samples, dim = N ** 3, 3
         used = 0x3F if cfg.cull_mode == 1 else 0x0F
-        halo = sum(bin(m & used).count("1") for m in masks) * N * N
-        total = n_chunks * samples + halo
-        ops = (n_chunks * samples * own_noise_ops(cfg) + halo * NOISE_EXEC_OPS["3d_table"]) * g.octaves
-        samples = total / n_chunks
+        total = n_chunks * N ** 3 + sum(bin(m & used).count("1") for m in masks) * N * N
     else:
         return None
-    achieved = ops / (ms_per_step / 1e3)
-    formula = total * g.octaves * NOISE_OPS[dim] / (ms_per_step / 1e3)
-    return {"samples_per_chunk": samples, "octaves": g.octaves,
-            "exec_ops_per_sample_octave": ops / (total * g.octaves),
-            "formula_ops_per_sample_octave": NOISE_OPS[dim],
-            "achieved_tops": achieved / 1e12, "peak_tops": FP32_OPS_NOMINAL / 1e12,
-            "peak_source": FP32_PEAK_SOURCE, "frac": achieved / FP32_OPS_NOMINAL,
-            "formula_tops": formula / 1e12,
-            "note": "executed lane operations of the step's noise over the whole step time (the "
-                    "launch also culls and emits); formula_tops counts the per-sample formula's "
-                    "operations at the same sample rate"}
+    return {"samples_per_chunk": total / n_chunks} | noise_rates(g.kind, total, g.octaves, ms_per_step / 1e3) | {
+        "note": "the noise's operations over the whole step time (the step also culls and emits)"}
 
 
 def cpu_baseline(wl, cfg, masks, seconds: float, threads: int = 0):
@@ -441,8 +433,10 @@ def measure_fused(name, args, torch, stream, flush, world=1, rank=0, local=0, he
     achieved = alg_bytes / (kernel_ms / 1e3) / 1e9
     kname = {"phased": "k_mesh_batch_phased", "overlap": "k_mesh_batch_overlap"}.get(
         run.tuning.get("schedule"), "k_mesh_batch")
+    if kname == "k_mesh_batch_overlap" and run.kernels_per_step > run.launches_per_step:
+        kname = "k_list_chunks + k_emit_lists"
     staged = run.tuning.get("halo") == "pool"
-    prof = NCU.get((kname + (" staged" if staged else ""), name))
+    prof = None if staged and "lists" in kname else NCU.get((kname + (" staged" if staged else ""), name))
     if staged:  # the step is the staged-halo sequence, the meshing kernel reading the pool
         kname += " (staged halo: coordinate map, neighbour lookup, k_generate into the pool)"
     roof = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak, "unit": "GB/s",
@@ -455,7 +449,7 @@ def measure_fused(name, args, torch, stream, flush, world=1, rank=0, local=0, he
         roof["traffic_source"] = (f"ncu dram__bytes_read.sum + dram__bytes_write.sum summed over one "
                                   f"step's kernels ({prof['summary']}), per step like achieved")
     elif prof:
-        per_launch_chunks = n / launches
+        per_launch_chunks = n / run.launches_per_step
         roof["traffic"] = prof["traffic"] * per_launch_chunks / prof["chunks"]
         roof["traffic_source"] = (f"ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch "
                                   f"({prof['summary']})"
@@ -474,10 +468,10 @@ def measure_fused(name, args, torch, stream, flush, world=1, rank=0, local=0, he
            "l2": "flushed before every step (256 MiB write, outside the events)",
            "roofline": roof, "clocks": clocks, "wall_s_timed_region": wall,
            "gpu_launches": steps * launches}
-    if prof and "warp_instructions" in prof and launches == 1:
+    if prof and "warp_instructions" in prof and (run.launches_per_step == 1 or prof.get("per_step")):
         instr = prof["warp_instructions"] * n / prof["chunks"]
         res["issue_roofline"] = {
-            "warp_instructions_per_launch": instr, "achieved": instr / (kernel_ms / 1e3),
+            "warp_instructions_per_step": instr, "achieved": instr / (kernel_ms / 1e3),
             "peak": ISSUE_PEAK, "unit": "warp instructions/s",
             "frac": instr / (kernel_ms / 1e3) / ISSUE_PEAK,
             "peak_source": "nominal (152 SMs x 4 schedulers x 2.07 GHz); instructions from "
@@ -560,14 +554,14 @@ def plain_per_chunk(ctx, wl, cfg, masks, stream, args, torch, limit):
 
 def noise_kernel(ctx, wl, cfg, stream, flush, args, torch):
     """The generation kernel alone (Chunk::new, src/chunk.rs:21-46): vox_generate writes the
-    occupancy of every chunk (no halo) to a device pool; its noise FP32 work is samples x
-    octaves x the formula's operation count, against the nominal FP32 instruction rate."""
+    occupancy of every chunk (no halo) to a device pool; its noise rate is samples x octaves x
+    the formula's operation count."""
     g = cfg.gen
     if g.kind not in (0, 1):
         return None
     n = len(wl.coords)
     N = cfg.chunk_size
-    samples, dim = (N * N, 2) if g.kind == 0 else (N ** 3, 3)
+    samples = N * N if g.kind == 0 else N ** 3
     d_coords = torch.tensor(list(wl.coords), dtype=torch.int32, device="cuda")
     pool = torch.empty(n * ctx.sizes.occ_words_per_chunk, dtype=torch.int32, device="cuda")
     steps = max(3, (args.suite_steps or args.steps) // 4)
@@ -579,21 +573,14 @@ def noise_kernel(ctx, wl, cfg, stream, flush, args, torch):
                              steps, stream, flush, torch)
     assert ctx.sync(raise_on_error=False) == 0
     ms = statistics.median(step_ms)
-    ops = n * samples * g.octaves * own_noise_ops(cfg)
-    achieved = ops / (ms / 1e3)
     return {"kernel": "k_generate", "ms": ms, "steps": steps, "chunks": n,
-            "samples_per_chunk": samples, "octaves": g.octaves,
-            "exec_ops_per_sample_octave": own_noise_ops(cfg),
-            "formula_ops_per_sample_octave": NOISE_OPS[dim], "achieved_tops": achieved / 1e12,
-            "peak_tops": FP32_OPS_NOMINAL / 1e12, "peak_source": FP32_PEAK_SOURCE,
-            "frac": achieved / FP32_OPS_NOMINAL,
-            "formula_tops": n * samples * g.octaves * NOISE_OPS[dim] / (ms / 1e3) / 1e12,
+            "samples_per_chunk": samples} | noise_rates(g.kind, n * samples, g.octaves, ms / 1e3) | {
             "occupancy_bytes": n * ctx.sizes.occ_words_per_chunk * 4,
-            "bound": ("FP32 pipe (FMA pipe 64 % active under ncu, math_pipe_throttle the top stall: "
-                      "profiles/k_generate_density.md)" if g.kind == 1 else
-                      "latency: one wave of one-chunk CTAs, each evaluating its columns' fBm as "
-                      "chains of dependent permutation-table reads and writing 1 KiB; the FP32 "
-                      "fraction is not this kernel's bound"),
+            "bound": ("issue and the FP32 pipe of the chunks at the surface (69 % of issue slots under "
+                      "ncu: profiles/face_lists.md); chunks that the bounds decide cost a fill"
+                      if g.kind == 1 else
+                      "latency: one wave of one-chunk CTAs, each a table load, two barriers and its "
+                      "columns' fBm, writing 1 KiB; the FP32 fraction is not this kernel's bound"),
             "api": "vox_generate (occupancy to a device pool, L2 flushed before each step)"}
 
 
