@@ -43,3 +43,32 @@ def test_draw_list_matches_numpy(vox, oracle, count, layout):
     assert np.array_equal(got[:20 * len(at)].view(np.uint32).reshape(-1, 5), want)
     assert (got[20 * len(at):20 * count] == 7).all()
     ctx.close()
+
+
+@pytest.mark.parametrize("count", [200, 1024, 1025, 5000])
+def test_draw_list_in_a_recorded_graph(vox, count):
+    """A recorded call against a direct one, replayed after a larger call of the same context."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(count)
+    stream = torch.cuda.Stream()
+    ctx = vox.Context(vox.make_config(chunk_size=16), stream=stream.cuda_stream)
+    big = 400000
+    coords = to_dev(rng.integers(-60, 60, (big, 3)).astype(np.int32))
+    offs = to_dev(np.concatenate([[0], np.cumsum(rng.integers(0, 9, big))]).astype(np.uint64))
+    planes = vox.frustum_planes(vox.camera_matrix((8.0, 30.0, -4.0), (0.7, -0.2, 0.6)))
+    want, draws, many = (dev_bytes(20 * k, fill=7) for k in (count, count, big))
+    n_want, n_draws = dev_bytes(4), dev_bytes(4)
+    torch.cuda.synchronize()
+    ctx.draw_list(planes, coords, offs, count, want, n_want)
+    ctx.sync()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        ctx.draw_list(planes, coords, offs, count, draws, n_draws)
+    ctx.draw_list(planes, coords, offs, big, many, dev_bytes(4))
+    ctx.sync()
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(to_np(n_draws)[:4], to_np(n_want)[:4])  # (behind them nothing is written)
+    assert np.array_equal(to_np(draws)[:20 * count], to_np(want)[:20 * count])
+    ctx.close()

@@ -1156,11 +1156,18 @@ int vox_draw_list(vox_ctx* ctx, const float planes[24], const vox_chunk_coord* d
   Planes pl;
   std::memcpy(pl.p, planes, sizeof pl.p);
   int st;
-  if ((st = ensure_state(ctx, (size_t)draw_list_tiles(n))) != VOX_OK) return st;
-  if ((st = before_batch_launch(ctx)) != VOX_OK) return st;  // the list takes a look-back epoch
+  // A caller's graph outlives this call: what it records must not hold the context's look-back
+  // words, which a larger batch moves and other launches use.
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) cudaGetLastError();
+  const bool walk = capturing != cudaStreamCaptureStatusNone || draw_list_tiles(n) == 1;
+  if (!walk) {
+    if ((st = ensure_state(ctx, (size_t)draw_list_tiles(n))) != VOX_OK) return st;
+    if ((st = before_batch_launch(ctx)) != VOX_OK) return st;  // the list takes a look-back epoch
+  }
   VOX_CUDA(ctx, launch_draw_list(pl, d_coords, reinterpret_cast<const unsigned long long*>(d_face_offsets),
                                  n, ctx->cfg.chunk_size, ctx->cfg.layout == VOX_LAYOUT_INSTANCED ? 1 : 0,
-                                 d_draws, d_count, ctx->d_ctl, ctx->d_state, ctx->spin_limit, ctx->stream),
+                                 d_draws, d_count, ctx->d_ctl, ctx->d_state, ctx->spin_limit, walk, ctx->stream),
            "draw list");
   return VOX_OK;
 }

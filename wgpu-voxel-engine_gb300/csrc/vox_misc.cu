@@ -162,18 +162,23 @@ k_frustum(Planes pl, const vox_chunk_coord* __restrict__ coords, int n, int exte
 // ERR_CAPACITY and are zeroed. Frustum test and list of 50,000 chunks 91 -> 12.8 us, of 8,000 20.5
 // -> 12.7 us with one CTA walking all tiles before; both are now bound by the two calls (up to
 // 2,000 chunks they were before, too).
-constexpr int kDrawTile = 256;
-__global__ void __launch_bounds__(kDrawTile)
+// A grid of one CTA (of kDrawWalk threads) walks the tiles by itself and touches neither the
+// tickets nor the look-back words: the form of a call that a caller's graph records, whose
+// replays must not depend on scratch that a later call may move or that other work uses.
+constexpr int kDrawTile = 256, kDrawWalk = 1024;
+__global__ void __launch_bounds__(kDrawWalk)
 k_draw_list(Planes pl, const vox_chunk_coord* __restrict__ coords,
             const unsigned long long* __restrict__ offs, int n, int extent, int instanced,
             DrawRecord* __restrict__ out, uint32_t* __restrict__ count, BatchCtl* ctl,
             unsigned long long* state, int spin_limit) {
-  __shared__ uint32_t wsum[kDrawTile / 32];
+  __shared__ uint32_t wsum[kDrawWalk / 32];
   __shared__ unsigned s_tile, s_epoch;
   __shared__ uint32_t s_base;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int warps = (int)blockDim.x >> 5;
+  const bool walk = gridDim.x == 1u;
   pdl_wait();
-  if (t == 0) {
+  if (t == 0 && !walk) {
     const unsigned epoch = ld_relaxed_u32(&ctl->epoch);
     __threadfence();
     const unsigned k = atomicAdd(&ctl->next, 1u);
@@ -185,9 +190,12 @@ k_draw_list(Planes pl, const vox_chunk_coord* __restrict__ coords,
     s_tile = k;
   }
   __syncthreads();
-  const int tile = (int)s_tile;
-  {
-    const long long i = (long long)tile * kDrawTile + t;
+  const int tiles = walk ? (int)(((long long)n + blockDim.x - 1) / blockDim.x) : 1;
+  const int tile0 = walk ? 0 : (int)s_tile;
+  uint32_t walked = 0;  // warp 0: records of the tiles that this CTA has walked
+  if (tiles == 0 && t == 0) *count = 0u;
+  for (int tile = tile0; tile < tile0 + tiles; ++tile) {
+    const long long i = (long long)tile * blockDim.x + t;
     bool vis = false;
     unsigned long long f0 = 0, nf = 0;
     if (i < n) {
@@ -200,19 +208,21 @@ k_draw_list(Planes pl, const vox_chunk_coord* __restrict__ coords,
     if (lane == 0) wsum[warp] = (uint32_t)__popc(bal);
     __syncthreads();
     if (warp == 0) {
-      const uint32_t v = lane < kDrawTile / 32 ? wsum[lane] : 0u;
+      const uint32_t v = lane < warps ? wsum[lane] : 0u;
       uint32_t incl = v;
 #pragma unroll
-      for (int off = 1; off < kDrawTile / 32; off <<= 1) {
+      for (int off = 1; off < 32; off <<= 1) {
         const uint32_t u = __shfl_up_sync(0xffffffffu, incl, off);
         if (lane >= off) incl += u;
       }
-      if (lane < kDrawTile / 32) wsum[lane] = incl - v;
-      const uint32_t total = __shfl_sync(0xffffffffu, incl, kDrawTile / 32 - 1);
-      const unsigned long long excl = lookback(state, ctl, s_epoch, tile, total, spin_limit);
+      if (lane < warps) wsum[lane] = incl - v;
+      const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+      const uint32_t excl =
+          walk ? walked : (uint32_t)lookback(state, ctl, s_epoch, tile, total, spin_limit);
+      walked += total;
       if (lane == 0) {
-        s_base = (uint32_t)excl;
-        if (tile == (int)gridDim.x - 1) *count = (uint32_t)excl + total;
+        s_base = excl;
+        if (tile == (walk ? tiles : (int)gridDim.x) - 1) *count = excl + total;
       }
     }
     __syncthreads();
@@ -240,6 +250,7 @@ k_draw_list(Planes pl, const vox_chunk_coord* __restrict__ coords,
       }
       out[s_base + wsum[warp] + before] = r;
     }
+    if (walk) __syncthreads();  // wsum and s_base are read before the next tile writes them
   }
 }
 
@@ -306,13 +317,13 @@ int draw_list_tiles(int n) { return n > 0 ? (int)(((long long)n + kDrawTile - 1)
 cudaError_t launch_draw_list(const Planes& planes, const void* coords,
                              const unsigned long long* offs, int n, int extent, int instanced,
                              DrawRecord* out, uint32_t* count, BatchCtl* ctl, unsigned long long* state,
-                             int spin_limit, cudaStream_t st) {
+                             int spin_limit, bool walk, cudaStream_t st) {
   const Planes* pl = &planes;
   const vox_chunk_coord* c = static_cast<const vox_chunk_coord*>(coords);
   void* params[] = {const_cast<Planes*>(pl), &c, &offs, &n, &extent, &instanced, &out, &count, &ctl, &state,
                     &spin_limit};
-  return launch_dependent((const void*)k_draw_list, dim3((unsigned)draw_list_tiles(n)), dim3(kDrawTile),
-                          params, 0, st);
+  return launch_dependent((const void*)k_draw_list, dim3(walk ? 1u : (unsigned)draw_list_tiles(n)),
+                          dim3(walk ? kDrawWalk : kDrawTile), params, 0, st);
 }
 
 }  // namespace vox
