@@ -68,17 +68,6 @@ NCU = {
     ("k_mesh_batch_phased", "heightmap"): {
         "traffic": 6473984, "warp_instructions": 16886488, "chunks": 1024,
         "summary": "profiles/k_mesh_batch_phased_heightmap.md"},
-    ("k_mesh_batch_overlap", "density"): {
-        "traffic": 658092032, "warp_instructions": 707898692, "chunks": 4096,
-        "summary": "profiles/k_mesh_batch_overlap_density.md"},
-    # staged halos: the traffic of one step's whole sequence (coordinate map, neighbour
-    # lookup, k_generate, k_generate_planes, meshing from the pool)
-    ("k_mesh_batch_overlap staged", "density"): {
-        "traffic": 650796032, "chunks": 4096, "per_step": True,
-        "summary": "profiles/staged_halo_density.md"},
-    ("k_mesh_batch_phased staged", "density"): {
-        "traffic": 688578304, "chunks": 4096, "per_step": True,
-        "summary": "profiles/staged_halo_density.md"},
     ("k_mesh_batch_overlap", "stress"): {
         "traffic": 47944924160, "chunks": 1024, "scaled_from_chunks": 48,
         "summary": "profiles/k_mesh_batch_overlap_stress.md"},
