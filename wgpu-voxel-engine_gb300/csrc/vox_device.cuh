@@ -1373,7 +1373,8 @@ __device__ void gen_chunk(ChunkSmem<N, LAYOUT>& s, const GenDev& g, vox_chunk_co
 
 // Occupancy from global memory: own rows copied; halo rows taken from the neighbours'
 // boundary planes (nbr[d] == nullptr: not loaded, zero halo). Every thread issues all its loads
-// before it uses one, so the chunk costs one memory latency instead of one per plane.
+// before it uses one, so the chunk costs one memory latency instead of one per plane. Plain loads:
+// the launch that writes the occupancy may still run when this kernel starts (see vox_launch.h).
 template <int N, int LAYOUT, int T>
 __device__ __forceinline__ void load_chunk(ChunkSmem<N, LAYOUT>& s, const uint32_t* self,
                                            const uint32_t* const nbr[6], unsigned use_mask) {
@@ -1386,7 +1387,7 @@ __device__ __forceinline__ void load_chunk(ChunkSmem<N, LAYOUT>& s, const uint32
   const int t = threadIdx.x;
   uint32_t own[kMost], px[2][kPlane], pr = 0u;
 #pragma unroll
-  for (int k = 0; k < kMost; ++k) own[k] = __ldg(self + t + k * T);
+  for (int k = 0; k < kMost; ++k) own[k] = self[t + k * T];
   // x planes: bit (N - 1) (h = 0) or bit 0 (h = 1) of the neighbour's row (y, z)
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -1394,21 +1395,21 @@ __device__ __forceinline__ void load_chunk(ChunkSmem<N, LAYOUT>& s, const uint32
     constexpr int kLast = (N - 1) >> 5;
 #pragma unroll
     for (int k = 0; k < kPlane; ++k)
-      px[h][k] = nb ? __ldg(nb + (t + k * T) * W + (h == 0 ? kLast : 0)) >> (h == 0 ? (N - 1) & 31 : 0) : 0u;
+      px[h][k] = nb ? nb[(t + k * T) * W + (h == 0 ? kLast : 0)] >> (h == 0 ? (N - 1) & 31 : 0) : 0u;
   }
   // whole rows: -z: (y, N-1); +z: (y, 0); -y: (N-1, z); +y: (0, z)
   auto row_word = [&](int i) {
     const int h = 2 + i / kRow, a = (i % kRow) / W, w = i % W;
     const uint32_t* nb = ((use_mask >> h) & 1u) ? nbr[h] : nullptr;
     const int r = h == 2 ? a * N + (N - 1) : (h == 3 ? a * N : (h == 4 ? (N - 1) * N + a : a));
-    return nb ? __ldg(nb + r * W + w) : 0u;
+    return nb ? nb[r * W + w] : 0u;
   };
   if (t < 4 * kRow) pr = row_word(t);
 #pragma unroll
   for (int k = 0; k < kMost; ++k) occw[t + k * T] = own[k];
   for (int k = kMost; k < kOwn; k += kMost) {
 #pragma unroll
-    for (int j = 0; j < kMost; ++j) own[j] = __ldg(self + t + (k + j) * T);
+    for (int j = 0; j < kMost; ++j) own[j] = self[t + (k + j) * T];
 #pragma unroll
     for (int j = 0; j < kMost; ++j) occw[t + (k + j) * T] = own[j];
   }

@@ -6,6 +6,12 @@
 // kernels, about a microsecond each; a kernel that follows one without a trigger starts as usual.
 // A kernel whose dependent reads anything before its own pdl_wait triggers after pdl_wait itself
 // (or is launched without this attribute), so that everything ahead of both has ended by then.
+// What earlier launches write is read behind the wait by plain (or volatile, or acquiring) loads:
+// pdl_wait keeps those behind it. No __ldg and no `const __restrict__` pointer for such data: both
+// say that it does not change while the kernel runs, which is untrue of a kernel that starts
+// early, and let the compiler move the load ahead of the wait. (The other cached-load intrinsics
+// give the compiler no order either; they are used where the address depends on an acquired
+// value.) Data of the context that no launch writes, such as grad2, may be read by __ldg.
 #pragma once
 
 #include <cstring>

@@ -138,8 +138,7 @@ __device__ __forceinline__ bool frustum_contains(const Planes& pl, vox_chunk_coo
 // One lane per corner: the launch is as short as its longest chain of operations, and a lane
 // of eight corners takes eight times as many.
 __global__ void __launch_bounds__(256)
-k_frustum(Planes pl, const vox_chunk_coord* __restrict__ coords, int n, int extent,
-          uint8_t* __restrict__ visible) {
+k_frustum(Planes pl, const vox_chunk_coord* coords, int n, int extent, uint8_t* visible) {
   pdl_trigger();
   pdl_wait();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -167,10 +166,9 @@ k_frustum(Planes pl, const vox_chunk_coord* __restrict__ coords, int n, int exte
 // replays must not depend on scratch that a later call may move or that other work uses.
 constexpr int kDrawTile = 256, kDrawWalk = 1024;
 __global__ void __launch_bounds__(kDrawWalk)
-k_draw_list(Planes pl, const vox_chunk_coord* __restrict__ coords,
-            const unsigned long long* __restrict__ offs, int n, int extent, int instanced,
-            DrawRecord* __restrict__ out, uint32_t* __restrict__ count, BatchCtl* ctl,
-            unsigned long long* state, int spin_limit) {
+k_draw_list(Planes pl, const vox_chunk_coord* coords, const unsigned long long* offs, int n, int extent,
+            int instanced, DrawRecord* out, uint32_t* count, BatchCtl* ctl, unsigned long long* state,
+            int spin_limit) {
   __shared__ uint32_t wsum[kDrawWalk / 32];
   __shared__ unsigned s_tile, s_epoch;
   __shared__ uint32_t s_base;

@@ -236,7 +236,7 @@ k_raster_faces(RasterArgs a, unsigned long long* keys, TileList list) {
       // The length may run past the room, but not around: no warp adds to a full list or more
       // than its room, which is at most 2^18 (times every resident warp: below 2^32).
       unsigned base = list.cap;
-      if (lane == 0 && all <= list.cap && __ldcg(list.count) < list.cap) base = atomicAdd(list.count, all);
+      if (lane == 0 && all <= list.cap && *const_cast<volatile unsigned*>(list.count) < list.cap) base = atomicAdd(list.count, all);
       place += __shfl_sync(0xffffffffu, base, 0);
     }
     // a box whose tiles do not all fit is done here, its places in the list left empty
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(256)
 k_raster_tiles(RasterArgs a, unsigned long long* keys, TileList list) {
   pdl_trigger();
   pdl_wait();
-  const unsigned n = min(__ldcg(list.count), list.cap);
+  const unsigned n = min(*list.count, list.cap);
   const int lane = threadIdx.x & 31;
   for (unsigned e = blockIdx.x * 8u + (threadIdx.x >> 5); e < n; e += gridDim.x * 8u) {
     const uint2 tile = list.tiles[e];
