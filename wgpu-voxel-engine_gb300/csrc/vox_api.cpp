@@ -14,6 +14,7 @@
 #include <string>
 
 #include "voxgpu.h"
+#include "vox_epochs.h"
 #include "vox_kernels.h"
 #include "vox_launch.h"
 #include "vox_tables.h"
@@ -94,6 +95,7 @@ struct vox_ctx {
   unsigned* d_err_mirror = nullptr;  // its device address
   unsigned long long* d_state = nullptr;
   size_t state_cap = 0;
+  EpochWipe state_wipe;
   unsigned long long launches = 0;
   // buffers of the host-pointer entry point
   void* d_in = nullptr;
@@ -118,7 +120,7 @@ struct vox_graph {
   uint32_t* d_scratch = nullptr;          // phased: occupancy + halo spill (n chunks)
   uint32_t* d_counts = nullptr;           // phased: face totals (n)
   size_t state_bytes = 0;
-  unsigned long long wiped_at = 0;        // context launch count when d_state was zeroed
+  EpochWipe wipe;                         // by the context's launch count
   int launches = 1;                       // kernel launches per replay (slabs of the batch)
   HaloScratch halo;                       // staged-halo buffers of the captured batch
 };
@@ -333,15 +335,14 @@ int ensure_state(vox_ctx* ctx, size_t n) {
   VOX_CUDA(ctx, cudaMalloc(&ctx->d_state, bytes), "cudaMalloc(state)");
   VOX_CUDA(ctx, cudaMemsetAsync(ctx->d_state, 0, bytes, ctx->stream), "cudaMemsetAsync(state)");
   ctx->state_cap = cap;
+  ctx->state_wipe.wiped_at = ctx->launches;
   return VOX_OK;
 }
 
-// Look-back states are tagged with a 24-bit launch epoch. A launch advances it by one, and a
-// launch that timed out by at most two (the host moves a failed launch to a fresh epoch), so
-// a wipe every 2^22 launches comes well before a tag can repeat.
-constexpr unsigned long long kStateWipePeriod = 1ull << 22;
+// Look-back states are tagged with a 24-bit launch epoch (see vox_epochs.h); the host moves a
+// failed launch to a fresh one.
 int before_batch_launch(vox_ctx* ctx) {
-  if (ctx->launches > 0 && (ctx->launches & (kStateWipePeriod - 1)) == 0 && ctx->d_state) {
+  if (ctx->d_state && ctx->state_wipe.due(ctx->launches)) {
     VOX_CUDA(ctx, cudaMemsetAsync(ctx->d_state, 0,
                                   (size_t)state_words(ctx->state_cap) * sizeof(unsigned long long),
                                   ctx->stream),
@@ -1401,7 +1402,7 @@ int vox_graph_capture(vox_ctx* ctx, const vox_chunk_coord* d_coords, const uint8
     if ((e = cudaMalloc(&g->d_state, g->state_bytes)) != cudaSuccess ||
         (e = cudaMemsetAsync(g->d_state, 0, g->state_bytes, ctx->stream)) != cudaSuccess)
       return bail(cuda_fail(ctx, e, "cudaMalloc(graph state)"));
-    g->wiped_at = ctx->launches;
+    g->wipe.wiped_at = ctx->launches;
     a.state = g->d_state;
   }
   // the graph owns its staged-halo buffers too (allocated before the capture)
@@ -1440,10 +1441,8 @@ int vox_graph_launch(vox_graph* g) {
   std::lock_guard<std::mutex> lk(ctx->mu);
   ctx->launches += (unsigned long long)g->launches;
   // look-back states carry a 24-bit launch epoch: zero them before a tag can repeat
-  if (g->d_state && ctx->launches - g->wiped_at >= kStateWipePeriod) {
+  if (g->d_state && g->wipe.due(ctx->launches))
     VOX_CUDA(ctx, cudaMemsetAsync(g->d_state, 0, g->state_bytes, ctx->stream), "cudaMemsetAsync(state)");
-    g->wiped_at = ctx->launches;
-  }
   VOX_CUDA(ctx, cudaGraphLaunch(g->exec, ctx->stream), "cudaGraphLaunch");
   return VOX_OK;
 }
