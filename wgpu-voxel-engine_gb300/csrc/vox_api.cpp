@@ -97,6 +97,11 @@ struct vox_ctx {
   size_t state_cap = 0;
   EpochWipe state_wipe;
   unsigned long long launches = 0;
+  // draw lists: the tickets' word, then look-back words of draw_cap tiles; nothing else uses them
+  unsigned long long* d_draw = nullptr;
+  size_t draw_cap = 0;
+  EpochWipe draw_wipe;
+  unsigned long long draws = 0;  // draw lists issued over tiles: their epochs
   // buffers of the host-pointer entry point
   void* d_in = nullptr;
   size_t in_cap = 0;
@@ -336,6 +341,24 @@ int ensure_state(vox_ctx* ctx, size_t n) {
   VOX_CUDA(ctx, cudaMemsetAsync(ctx->d_state, 0, bytes, ctx->stream), "cudaMemsetAsync(state)");
   ctx->state_cap = cap;
   ctx->state_wipe.wiped_at = ctx->launches;
+  return VOX_OK;
+}
+
+// Look-back words of a draw list of `tiles` tiles. The old ones go once the new ones are there.
+int ensure_draw(vox_ctx* ctx, size_t tiles) {
+  if (tiles <= ctx->draw_cap) return VOX_OK;
+  const size_t cap = std::max<size_t>(tiles, 8192), bytes = (1 + cap) * sizeof(unsigned long long);
+  unsigned long long* words = nullptr;
+  VOX_CUDA(ctx, cudaMalloc(&words, bytes), "cudaMalloc(draw list)");
+  const cudaError_t e = cudaMemsetAsync(words, 0, bytes, ctx->stream);
+  if (e != cudaSuccess) {
+    cudaFree(words);
+    return cuda_fail(ctx, e, "cudaMemsetAsync(draw list)");
+  }
+  cudaFree(ctx->d_draw);  // (waits for the launches that use them)
+  ctx->d_draw = words;
+  ctx->draw_cap = cap;
+  ctx->draw_wipe.wiped_at = ctx->draws;
   return VOX_OK;
 }
 
@@ -762,7 +785,7 @@ int vox_ctx_create(const vox_config* cfg, void* stream, vox_ctx** out) {
     return cleanup(st);
   ctx->last_error.clear();
   // enough for every batch of 8192 chunks and every draw list of 2 million
-  if ((st = ensure_state(ctx, 8192)) != VOX_OK) return cleanup(st);
+  if ((st = ensure_state(ctx, 8192)) != VOX_OK || (st = ensure_draw(ctx, 8192)) != VOX_OK) return cleanup(st);
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return cleanup(VOX_ERR_CUDA);
   *out = ctx;
   return VOX_OK;
@@ -775,6 +798,7 @@ int vox_ctx_destroy(vox_ctx* ctx) {
   cudaFree(ctx->d_grad2);
   cudaFree(ctx->d_ctl);
   cudaFree(ctx->d_state);
+  cudaFree(ctx->d_draw);
   cudaFree(ctx->d_scratch);
   cudaFree(ctx->d_counts);
   cudaFree(ctx->d_in);
@@ -1156,19 +1180,28 @@ int vox_draw_list(vox_ctx* ctx, const float planes[24], const vox_chunk_coord* d
     return fail(ctx, VOX_ERR_INVALID, "bad arguments");
   Planes pl;
   std::memcpy(pl.p, planes, sizeof pl.p);
-  int st;
-  // A caller's graph outlives this call: what it records must not hold the context's look-back
-  // words, which a larger batch moves and other launches use.
+  // A caller's graph outlives this call: what it records must not hold the look-back words, which a
+  // larger list moves and other lists use. One CTA also walks the list where there is no room
+  // for the words.
+  const int tiles = draw_list_tiles(n);
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) cudaGetLastError();
-  const bool walk = capturing != cudaStreamCaptureStatusNone || draw_list_tiles(n) == 1;
+  bool walk = capturing != cudaStreamCaptureStatusNone || tiles == 1;
+  if (!walk && ensure_draw(ctx, (size_t)tiles) != VOX_OK) {
+    cudaGetLastError();
+    walk = true;
+  }
+  unsigned epoch = 0;
   if (!walk) {
-    if ((st = ensure_state(ctx, (size_t)draw_list_tiles(n))) != VOX_OK) return st;
-    if ((st = before_batch_launch(ctx)) != VOX_OK) return st;  // the list takes a look-back epoch
+    if (ctx->draw_wipe.due(ctx->draws))
+      VOX_CUDA(ctx, cudaMemsetAsync(ctx->d_draw, 0, (1 + ctx->draw_cap) * sizeof(unsigned long long), ctx->stream),
+               "cudaMemsetAsync(draw list)");
+    epoch = (unsigned)ctx->draws++;
   }
   VOX_CUDA(ctx, launch_draw_list(pl, d_coords, reinterpret_cast<const unsigned long long*>(d_face_offsets),
                                  n, ctx->cfg.chunk_size, ctx->cfg.layout == VOX_LAYOUT_INSTANCED ? 1 : 0,
-                                 d_draws, d_count, ctx->d_ctl, ctx->d_state, ctx->spin_limit, walk, ctx->stream),
+                                 d_draws, d_count, ctx->d_ctl, walk ? nullptr : ctx->d_draw, epoch,
+                                 ctx->spin_limit, ctx->stream),
            "draw list");
   return VOX_OK;
 }

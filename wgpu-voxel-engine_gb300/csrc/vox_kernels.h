@@ -57,13 +57,13 @@ struct RasterArgs {
 cudaError_t launch_raster(const RasterArgs& a, unsigned long long* keys, uint8_t* rgba,
                           cudaStream_t st);
 struct BatchCtl;
-// The draw list of n chunks; state: look-back words of draw_list_tiles(n) tiles. walk: one CTA
-// walks the tiles and uses no state.
+// The draw list of n chunks. words: a tickets' word, zero between launches, then look-back words of
+// draw_list_tiles(n) tiles, tagged with `epoch`; null: one CTA walks the tiles and uses none.
 int draw_list_tiles(int n);
 cudaError_t launch_draw_list(const Planes& planes, const void* coords,
                              const unsigned long long* offs, int n, int extent, int instanced,
-                             DrawRecord* out, uint32_t* count, BatchCtl* ctl, unsigned long long* state,
-                             int spin_limit, bool walk, cudaStream_t st);
+                             DrawRecord* out, uint32_t* count, BatchCtl* ctl, unsigned long long* words,
+                             unsigned epoch, int spin_limit, cudaStream_t st);
 
 // Neighbour lookup of the staged-halo path (vox_halo.cu): a hash map of the batch's
 // coordinates (cap_mask + 1 slots, a power of two at least twice n), then per chunk and

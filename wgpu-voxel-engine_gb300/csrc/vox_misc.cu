@@ -161,31 +161,27 @@ k_frustum(Planes pl, const vox_chunk_coord* coords, int n, int extent, uint8_t* 
 // ERR_CAPACITY and are zeroed. Frustum test and list of 50,000 chunks 91 -> 12.8 us, of 8,000 20.5
 // -> 12.7 us with one CTA walking all tiles before; both are now bound by the two calls (up to
 // 2,000 chunks they were before, too).
-// A grid of one CTA (of kDrawWalk threads) walks the tiles by itself and touches neither the
-// tickets nor the look-back words: the form of a call that a caller's graph records, whose
-// replays must not depend on scratch that a later call may move or that other work uses.
+// Tickets and look-back words are the draw lists' own, and the epoch is the host's count of them
+// (they are issued in stream order), so that a list is independent of batches: of one that a
+// caller's graph replays on another stream, and of one that gave up with its queue words mid-way.
+// Without words one CTA (of kDrawWalk threads) walks the tiles by itself: the form of a call that
+// a caller's graph records, whose replays must not depend on scratch that a later call may move.
 constexpr int kDrawTile = 256, kDrawWalk = 1024;
 __global__ void __launch_bounds__(kDrawWalk)
 k_draw_list(Planes pl, const vox_chunk_coord* coords, const unsigned long long* offs, int n, int extent,
-            int instanced, DrawRecord* out, uint32_t* count, BatchCtl* ctl, unsigned long long* state,
-            int spin_limit) {
+            int instanced, DrawRecord* out, uint32_t* count, BatchCtl* ctl, unsigned long long* words,
+            unsigned epoch, int spin_limit) {
   __shared__ uint32_t wsum[kDrawWalk / 32];
-  __shared__ unsigned s_tile, s_epoch;
+  __shared__ unsigned s_tile;
   __shared__ uint32_t s_base;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int warps = (int)blockDim.x >> 5;
-  const bool walk = gridDim.x == 1u;
+  const bool walk = words == nullptr;
   pdl_wait();
   if (t == 0 && !walk) {
-    const unsigned epoch = ld_relaxed_u32(&ctl->epoch);
-    __threadfence();
-    const unsigned k = atomicAdd(&ctl->next, 1u);
-    if (k == gridDim.x - 1u) {  // the last ticket: every CTA has read the epoch
-      ctl->next = 0u;
-      ctl->epoch = epoch + 1u;
-    }
-    s_epoch = epoch;
-    s_tile = k;
+    unsigned* tickets = reinterpret_cast<unsigned*>(words);
+    s_tile = atomicAdd(tickets, 1u);
+    if (s_tile == gridDim.x - 1u) *tickets = 0u;  // the last one
   }
   __syncthreads();
   const int tiles = walk ? (int)(((long long)n + blockDim.x - 1) / blockDim.x) : 1;
@@ -216,7 +212,7 @@ k_draw_list(Planes pl, const vox_chunk_coord* coords, const unsigned long long* 
       if (lane < warps) wsum[lane] = incl - v;
       const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
       const uint32_t excl =
-          walk ? walked : (uint32_t)lookback(state, ctl, s_epoch, tile, total, spin_limit);
+          walk ? walked : (uint32_t)lookback(words + 1, ctl, epoch, tile, total, spin_limit);
       walked += total;
       if (lane == 0) {
         s_base = excl;
@@ -314,14 +310,14 @@ int draw_list_tiles(int n) { return n > 0 ? (int)(((long long)n + kDrawTile - 1)
 
 cudaError_t launch_draw_list(const Planes& planes, const void* coords,
                              const unsigned long long* offs, int n, int extent, int instanced,
-                             DrawRecord* out, uint32_t* count, BatchCtl* ctl, unsigned long long* state,
-                             int spin_limit, bool walk, cudaStream_t st) {
+                             DrawRecord* out, uint32_t* count, BatchCtl* ctl, unsigned long long* words,
+                             unsigned epoch, int spin_limit, cudaStream_t st) {
   const Planes* pl = &planes;
   const vox_chunk_coord* c = static_cast<const vox_chunk_coord*>(coords);
-  void* params[] = {const_cast<Planes*>(pl), &c, &offs, &n, &extent, &instanced, &out, &count, &ctl, &state,
-                    &spin_limit};
-  return launch_dependent((const void*)k_draw_list, dim3(walk ? 1u : (unsigned)draw_list_tiles(n)),
-                          dim3(walk ? kDrawWalk : kDrawTile), params, 0, st);
+  void* params[] = {const_cast<Planes*>(pl), &c, &offs, &n, &extent, &instanced, &out, &count, &ctl, &words,
+                    &epoch, &spin_limit};
+  return launch_dependent((const void*)k_draw_list, dim3(words ? (unsigned)draw_list_tiles(n) : 1u),
+                          dim3(words ? kDrawTile : kDrawWalk), params, 0, st);
 }
 
 }  // namespace vox
