@@ -17,6 +17,7 @@
 #include "vox_epochs.h"
 #include "vox_kernels.h"
 #include "vox_launch.h"
+#include "vox_scratch.h"
 #include "vox_tables.h"
 #include "vox_trace.h"
 #include "vox_types.h"
@@ -83,9 +84,9 @@ struct vox_ctx {
   int emit_grid = 0;                  // persistent grid of the list emission
   int host_grid[4] = {0, 0, 0, 0};    // grid of launches that write host memory (staged)
   // phased and overlap schedules: per-chunk occupancy + halo spill and face totals
-  uint32_t* d_scratch = nullptr;
+  ScratchBuffer scratch;
   uint32_t* d_counts = nullptr;
-  size_t scratch_bytes = 0, counts_cap = 0;
+  size_t counts_cap = 0;
   TablesDev* d_tables = nullptr;
   float2* d_grad2 = nullptr;
   TablesDev h_tables{};  // the fused batch kernels take the tables as a kernel parameter
@@ -309,16 +310,20 @@ size_t slot_bytes(const vox_ctx* ctx, bool lists) {
   return (size_t)(lists ? ctx->ks->list_slot_bytes : ctx->ks->spill_bytes);
 }
 
-// Per-chunk scratch and face totals for n chunks (grow; never shrink).
-int ensure_scratch(vox_ctx* ctx, size_t n, size_t slot) {
+// Per-chunk scratch and face totals for n chunks (grow; never shrink). Clears `lists` where only the
+// persistent launch's slots fit (64^3 lists take twice their room).
+int ensure_scratch(vox_ctx* ctx, size_t n, bool& lists) {
   const size_t cap = std::max<size_t>(n, 1024);
-  if (n * slot > ctx->scratch_bytes) {
-    cudaFree(ctx->d_scratch);
-    ctx->d_scratch = nullptr;
-    ctx->scratch_bytes = 0;
-    VOX_CUDA(ctx, cudaMalloc(&ctx->d_scratch, cap * slot), "cudaMalloc(scratch)");
-    ctx->scratch_bytes = cap * slot;
-  }
+  const int e = grow_scratch(
+      ctx->scratch, n, slot_bytes(ctx, true), slot_bytes(ctx, false), 1024 * slot_bytes(ctx, false), lists,
+      (int)cudaErrorMemoryAllocation,
+      [](size_t bytes, void** out) {
+        const cudaError_t err = cudaMalloc(out, bytes);
+        if (err == cudaErrorMemoryAllocation) cudaGetLastError();
+        return (int)err;
+      },
+      [](void* p) { cudaFree(p); });
+  if (e != 0) return cuda_fail(ctx, (cudaError_t)e, "cudaMalloc(scratch)");
   if (n > ctx->counts_cap) {
     cudaFree(ctx->d_counts);
     ctx->d_counts = nullptr;
@@ -385,8 +390,6 @@ MeshArgs base_args(vox_ctx* ctx) {
   a.full6 = ctx->cfg.cull_mode == VOX_CULL_FULL6 ? 1 : 0;
   a.stage_faces = ctx->stage_faces;
   a.spin_limit = ctx->spin_limit;
-  a.scratch = ctx->d_scratch;
-  a.counts = ctx->d_counts;
   return a;
 }
 
@@ -624,14 +627,8 @@ int batch_launch(vox_ctx* ctx, MeshArgs& a, int gm, bool host_out = false) {
   const int slab = slab_of(ctx, a.n);
   bool lists = use_lists(ctx, gm, slab, host_out);
   if (ctx->schedule != VOX_SCHEDULE_LOOKBACK) {  // the spill slots of phases A and C
-    st = ensure_scratch(ctx, (size_t)slab, slot_bytes(ctx, lists));
-    if (st == VOX_ERR_OOM && lists && ctx->ks->list_slot_bytes > ctx->ks->spill_bytes) {
-      cudaGetLastError();  // 64^3 lists take twice the room of the persistent launch's slots
-      lists = false;
-      st = ensure_scratch(ctx, (size_t)slab, slot_bytes(ctx, lists));
-    }
-    if (st != VOX_OK) return st;
-    a.scratch = ctx->d_scratch;
+    if ((st = ensure_scratch(ctx, (size_t)slab, lists)) != VOX_OK) return st;
+    a.scratch = static_cast<uint32_t*>(ctx->scratch.data);
     a.counts = ctx->d_counts;
   }
   if (ctx->schedule != VOX_SCHEDULE_PHASED) {  // look-back state words
@@ -799,7 +796,7 @@ int vox_ctx_destroy(vox_ctx* ctx) {
   cudaFree(ctx->d_ctl);
   cudaFree(ctx->d_state);
   cudaFree(ctx->d_draw);
-  cudaFree(ctx->d_scratch);
+  cudaFree(ctx->scratch.data);
   cudaFree(ctx->d_counts);
   cudaFree(ctx->d_in);
   cudaFree(ctx->d_offsets);
