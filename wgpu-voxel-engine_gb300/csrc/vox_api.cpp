@@ -290,10 +290,13 @@ bool default_shape(const vox_ctx* ctx, int topt, int stage_faces, int ctas_per_s
 // Whether a launch of n chunks goes through the face lists (vox_lists.cuh): the overlap schedule
 // with the default shape and outputs in device memory, unless the voxels are random, whose
 // chunks never fit a list. Large batches of small heightmap chunks in the vertex layout stay
-// with the persistent launch: from two rounds of list CTAs on (2432 chunks of 16^3, 9728 of
-// 8^3) emission that overlaps generation from the start is worth more than occupancy. us a
-// batch, lists / one launch: 16^3 2000 chunks 50 / 52, 3000 69 / 71 (128 threads: 66), 4000
-// 93 / 91 (85), 8000 181 / 171 (153); 8^3 4000 38 / 46, 16000 108 / 101. Lists stay ahead for
+// with the persistent launch, whose emission overlaps generation from the start: beyond three rounds
+// of list CTAs of 16^3 (3648 chunks), and beyond 5/4 rounds of 8^3 (6080 chunks). us a batch, lists /
+// one launch, terrain of four octaves and of one: 16^3 1500 chunks 40.0 / 39.8 and 36.0 / 38.3, 2000
+// 48.0 / 50.2 and 44.5 / 47.7, 3000 67.9 / 70.9 and 64.8 / 67.0, 3600 81.2 / 82.9 and 74.5 / 78.9, 4000
+// 91.6 / 90.5 and 90.1 / 86.6; 8^3 4000 36.7 / 42.6 and 36.1 / 39.3, 6000 47.6 / 49.3 and 47.9 / 45.9,
+// 8000 58.5 / 57.9 and 60.5 / 56.3, 16000 104.9 / 99.9 and 109.5 / 96.6. (CTAs of 128 threads take 16^3
+// terrain further, which is the tuner's to find: 3000 chunks 65.9, 8000 151.) Lists stay ahead for
 // instances (16^3, 8000 chunks 126 / 156), caves (16^3, 4000 chunks 104 / 113) and from 32^3 on
 // (terrain, 4096 chunks 320 / 344).
 bool use_lists(const vox_ctx* ctx, int gm, int n, bool host_out) {
@@ -302,7 +305,7 @@ bool use_lists(const vox_ctx* ctx, int gm, int n, bool host_out) {
     return false;
   const int N = ctx->cfg.chunk_size;
   return N > 16 || gm != GM_HEIGHT || ctx->cfg.layout != VOX_LAYOUT_VERTEX ||
-         n <= 2 * ctx->num_sms * (N == 16 ? 8 : 32);
+         n <= ctx->num_sms * (N == 16 ? 3 * 8 : 5 * 32 / 4);
 }
 
 // Scratch of one chunk of a launch.
@@ -829,6 +832,7 @@ static int sync_locked(vox_ctx* ctx) {
     ctx->h_ctl->next = 0;
     ctx->h_ctl->next_scan = 0;
     ctx->h_ctl->done = 0;
+    ctx->h_ctl->open = 0;
     ctx->h_ctl->bar_count = 0;
     ctx->h_ctl->epoch += 1;
   }

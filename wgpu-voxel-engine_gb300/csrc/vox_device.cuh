@@ -2091,9 +2091,18 @@ __device__ void emit_chunk_direct(const ChunkSmem<N, LAYOUT>& s, vox_chunk_coord
 // order, in the chunk's spill slot, written by the generation item from the face voxels and
 // read by the emission item, which then needs no chunk state in shared memory, no compaction
 // and no barrier beyond the offset's. It takes 4 bytes a face next to the 68 or 120 it
-// describes. Chunks with more faces than the slot holds, kMiscOff / 4 (7 N^2 to 10 N^2 up to
-// 32^3, 3.7 N^2 at 64^3; terrain has 2 N^2 to 4 N^2, random voxels 100 N^2), spill their
-// occupancy and row lists instead and are compacted at emission.
+// describes. Chunks with more faces than max_list_faces (3.7 N^2 at 64^3, whose slots hold no
+// more) spill their occupancy and row lists instead and are compacted at emission.
+//
+// The most faces of a list in a slot of `bytes`: what fits, but no more than `most` N^2, from where its
+// traffic costs more than the compaction: 9 at 16^3 (white-noise columns of 11 N^2 faces, 2000 chunks:
+// 151 us a batch in one launch with lists of all that fits, 138 without; 155 and 137 in two) and in one
+// launch 5 at 8^3 (8000 chunks of 6 N^2: 107 and 100 us; in two launches lists stay ahead, 50 us of
+// 3000 chunks against 59). Terrain has 2 N^2 to 4 N^2 faces, random voxels 6 N^2 to 100 N^2.
+template <int N>
+__host__ __device__ constexpr uint32_t max_list_faces(int bytes, int most) {
+  return (uint32_t)(bytes / 4 < most * N * N ? bytes / 4 : most * N * N);
+}
 // Position of set bit n (from 0) of m, which has more than n.
 template <int N, typename RowT>
 __device__ __forceinline__ int nth_bit(RowT m, int n) {
@@ -2611,7 +2620,7 @@ k_mesh_batch_overlap(const __grid_constant__ MeshArgs a, const __grid_constant__
   constexpr int kVlOff = kNzOff + P::kNz;
   constexpr int kMiscOff = kVlOff + P::kVList;
   static_assert(P::kSpill == kMiscOff + P::kMisc, "spill layout");
-  constexpr uint32_t kListCap = kMiscOff / 4;  // faces of a face list (see write_face_list)
+  constexpr uint32_t kListCap = max_list_faces<N>(kMiscOff, N == 8 ? 5 : 9);  // faces of a face list
   constexpr int kListed = -2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ChunkSmem<N, LAYOUT> s;

@@ -23,9 +23,9 @@
 
 namespace vox {
 
-// Slot of a chunk in the scratch: its face list, or (more faces than the list holds) the spilled
-// chunk state of SmemPlan. The list holds 7 N^2 to 10 N^2 faces up to 32^3 (the size of
-// the chunk state) and 8 N^2 at 64^3; terrain has 2 N^2 to 4 N^2, random voxels 100 N^2.
+// Slot of a chunk in the scratch: its face list, or (more than kCap faces) the spilled chunk state of
+// SmemPlan. 64^3 slots hold a list of 8 N^2 faces, the others the size of the chunk state (see
+// max_list_faces).
 template <int N>
 struct ListSlot {
   using P = SmemPlan<N, VOX_LAYOUT_VERTEX>;
@@ -33,9 +33,13 @@ struct ListSlot {
   static constexpr int kVlOff = kNzOff + P::kNz;
   static constexpr int kMiscOff = kVlOff + P::kVList;
   static constexpr int kBytes = N == 64 ? 8 * N * N * 4 : P::kSpill;
-  static constexpr uint32_t kCap = kBytes / 4;
+  static constexpr uint32_t kCap = max_list_faces<N>(kBytes, N == 8 ? 10 : 9);
   static_assert(kBytes >= P::kSpill, "the slot holds a spilled chunk state");
 };
+
+// a.counts[i] of a chunk that has no list counts the runs of it that emission warps have taken; all
+// are taken once it is at least kTaken, as those of a listed chunk are from the start.
+constexpr uint32_t kTaken = 1u << 30;
 
 // CTA sizes of k_list_chunks: kBig = 0 for many chunks; kBig = 1, up to one thread a row, for
 // batches of no more chunks than SMs, where a chunk's latency is the batch's.
@@ -105,6 +109,10 @@ k_list_chunks(const __grid_constant__ MeshArgs a, const __grid_constant__ Tables
   s.stage = lists + M::kLists;
   const uint32_t total = count_and_scan<N, VOX_LAYOUT_VERTEX, T>(s);
   unsigned char* dst = reinterpret_cast<unsigned char*>(a.scratch) + (unsigned long long)i * S::kBytes;
+  if (t == 0) {
+    __stcg(a.counts + i, total <= S::kCap ? kTaken : 0u);
+    if (total > S::kCap) atomicAdd(&a.ctl->open, 1u);
+  }
   if (total <= S::kCap) {
     write_face_list<N, VOX_LAYOUT_VERTEX>(s, reinterpret_cast<uint32_t*>(dst));
   } else {
@@ -241,6 +249,13 @@ struct Origin {
   }
 };
 
+// A store of records; kStream: as the first to leave L2, for outputs that do not fit there.
+template <bool kStream, typename T>
+__device__ __forceinline__ void put(T* p, T v) {
+  if (kStream) __stcs(p, v);
+  else *p = v;
+}
+
 // kPad: staging and table entries spread over the banks (41.2 -> 39.5 us on the cave chunks of
 // 32^3; at 16^3 the shorter address arithmetic is worth more, 33.4 against 34.0 us).
 template <int LAYOUT, bool kPad>
@@ -272,7 +287,7 @@ struct FaceStore<VOX_LAYOUT_VERTEX, kPad> {
   }
 
   // Writes nw faces (chunk-local indices first, first + 1, ...) at global face g.
-  template <bool kSmall>
+  template <bool kSmall, bool kStream = false>
   __device__ __forceinline__ void batch(uint32_t q, int nw, uint32_t first, const Origin& org,
                                         unsigned long long g, void* out0, void* out1) const {
     const float4* C = table + (q >> 24) * (unsigned)kEntry;
@@ -293,14 +308,14 @@ struct FaceStore<VOX_LAYOUT_VERTEX, kPad> {
     const int units = nw * 6;
 #pragma unroll
     for (int k = 0; k < 6; ++k)
-      if (32 * k + lane < units) o[32 * k] = buf[32 * k + lane + (kPad ? (32 * k + lane) / 24 : 0)];
+      if (32 * k + lane < units) put<kStream>(o + 32 * k, buf[32 * k + lane + (kPad ? (32 * k + lane) / 24 : 0)]);
     // indices 4 f + {0, 2, 1, 3, 1, 2}: 8-byte pair j of face u / 3
     uint2* x = reinterpret_cast<uint2*>(reinterpret_cast<unsigned char*>(out1) + g * 24ull) + lane;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const int u = 32 * k + lane, f = u / 3, j = u - 3 * f;
       const uint32_t b = 4u * (first + (uint32_t)f);
-      if (f < nw) x[32 * k] = make_uint2(b + (j == 0 ? 0u : 1u), b + (j == 1 ? 3u : 2u));
+      if (f < nw) put<kStream>(x + 32 * k, make_uint2(b + (j == 0 ? 0u : 1u), b + (j == 1 ? 3u : 2u)));
     }
   }
 };
@@ -327,7 +342,7 @@ struct FaceStore<VOX_LAYOUT_INSTANCED, kPad> {
     }
   }
 
-  template <bool kSmall>
+  template <bool kSmall, bool kStream = false>
   __device__ __forceinline__ void batch(uint32_t q, int nw, uint32_t, const Origin& org,
                                         unsigned long long g, void* out0, void*) const {
     const float4* M = reinterpret_cast<const float4*>(table + (q >> 24) * 20u);
@@ -356,14 +371,42 @@ struct FaceStore<VOX_LAYOUT_INSTANCED, kPad> {
 #pragma unroll
       for (int k = 0; k < 5; ++k)
         if (32 * k + lane < units)
-          reinterpret_cast<float4*>(o)[32 * k + lane] = reinterpret_cast<const float4*>(buf)[32 * k + lane];
+          put<kStream>(reinterpret_cast<float4*>(o) + 32 * k + lane, reinterpret_cast<const float4*>(buf)[32 * k + lane]);
       if (lane < (nw * 17 & 3))
-        reinterpret_cast<float*>(o)[4 * units + lane] = buf[4 * units + lane];
+        put<kStream>(reinterpret_cast<float*>(o) + 4 * units + lane, buf[4 * units + lane]);
     } else {
-      for (int k = lane; k < nw * 17; k += 32) reinterpret_cast<float*>(o)[k] = buf[k];
+      for (int k = lane; k < nw * 17; k += 32) put<kStream>(reinterpret_cast<float*>(o) + k, buf[k]);
     }
   }
 };
+
+// A chunk without a list is emitted by compaction from its spilled state, in runs of run_groups()
+// groups of 32 elements that warps take one at a time. Such chunks are dense, and a batch of them is
+// bound by HBM writes and by its last wave: 2000 chunks of 16^3 in four parts are 1.6 waves of warps,
+// which left a third of the warps idle in the second. So the warps of a chunk's parts share its runs,
+// and a warp that has no part left, and has met such chunks, looks for others with runs left: chunk
+// open_chunk() from `from` on, in steps of 32 counts (done: how many are behind it), or -1. Their
+// records leave L2 first (__stcs), as their batches do not fit there. us a batch, one part a warp with
+// plain stores -> now (one launch before the lists): random voxels from a pool, 2000 chunks of 16^3
+// 332 -> 259 (269), 400 of 32^3 431 -> 382 (385); white-noise columns, 2000 of 16^3 171 -> 137 (138,
+// with the shorter list below), 400 of 32^3 237 -> 210 (209); white-noise density, 2000 of 16^3 329 ->
+// 288 (312), 400 of 32^3 515 -> 446 (473).
+template <int N>
+__host__ __device__ constexpr int run_groups() { return N <= 16 ? 4 : 8; }
+
+static __device__ int open_chunk(const MeshArgs& a, int from, unsigned& done, unsigned turn) {
+  const int lane = threadIdx.x & 31;
+  for (; done < (unsigned)a.n && ld_relaxed_u32(&a.ctl->open) != 0u; done += 32u) {
+    const long long at = (long long)from + done + lane;
+    const int i = (int)(at < a.n ? at : at - a.n);
+    const unsigned left =
+        __ballot_sync(0xffffffffu, done + lane < (unsigned)a.n && ld_relaxed_u32(a.counts + i) < kTaken);
+    if (left == 0u) continue;
+    const unsigned ahead = left & (0xffffffffu << (turn & 31u));  // (warps begin at different ones)
+    return __shfl_sync(0xffffffffu, i, __ffs(ahead != 0u ? ahead : left) - 1);
+  }
+  return -1;
+}
 
 template <int N, int LAYOUT>
 __global__ void __launch_bounds__(emit_threads<N>(), 1024 / emit_threads<N>())
@@ -400,26 +443,38 @@ k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
     }
   }
   // Emission items: part k % 2^split of chunk k >> split, dealt out to the warps of the grid in
-  // chunk order.
+  // chunk order; then runs of chunks without a list.
+  // (32-bit: a chunk's scratch is more than 2 KB, so no launch has 2^32 items.)
   const unsigned parts = 1u << a.split;
-  const unsigned long long items = (unsigned long long)a.n << a.split;
-  for (unsigned long long k = (unsigned long long)blockIdx.x * (kEmitThreads / 32) + warp;
-       ok && k < items; k += (unsigned long long)gridDim.x * (kEmitThreads / 32)) {
-    const int i = (int)(k >> a.split);
-    const unsigned part = (unsigned)k & (parts - 1u);
+  const unsigned items = (unsigned)a.n << a.split, stride = gridDim.x * (kEmitThreads / 32);
+  unsigned k = blockIdx.x * (kEmitThreads / 32) + (unsigned)warp;
+  int met = -1;  // the last chunk without a list that this warp has met
+  unsigned done = 0;
+  while (ok) {
+    int i = (int)(k >> a.split);
+    const unsigned part = k & (parts - 1u);
+    if (k < items) {
+      k += stride;
+    } else {
+      if (met < 0) break;
+      i = open_chunk(a, met, done, k);
+      if (i < 0) break;
+    }
     const vox_chunk_coord c = a.coords[i];
     unsigned long long g0;
     unsigned total;
-    ok = chunk_offset(a, epoch, i, g0, total);
+    // (from 32^3 on epoch and base are read again for each item, which spares the registers: the
+    // cave rebuild of 777 chunks 35.6 -> 35.0 us; at 16^3 it costs as much)
+    ok = chunk_offset(a, N > 16 ? *const_cast<volatile unsigned*>(&s_epoch) : epoch, i, g0, total);
     if (!ok || total == 0u) continue;
-    g0 += base0;
+    g0 += N > 16 ? *const_cast<volatile unsigned long long*>(&s_base0) : base0;
     const Origin org(c, N);
     auto send = [&](uint32_t q, int nw, uint32_t first, unsigned long long g) {
       if (org.small) store.template batch<true>(q, nw, first, org, g, a.out0, a.out1);
       else store.template batch<false>(q, nw, first, org, g, a.out0, a.out1);
     };
     unsigned char* src = reinterpret_cast<unsigned char*>(a.scratch) + (unsigned long long)i * S::kBytes;
-    if (total <= S::kCap) {
+    if (total <= S::kCap) {  // (never of an open chunk)
       // the output lines that the chunk touches, cut evenly over the parts
       const uint32_t* codes = reinterpret_cast<const uint32_t*>(src);
       const unsigned phase = (unsigned)(g0 & (unsigned long long)(kLine - 1u));
@@ -443,7 +498,8 @@ k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
         cnt = cnt2;
         q = q2;
       }
-    } else {  // no list: compaction from the spilled chunk state
+    } else {
+      met = i;
       ChunkSmem<N, LAYOUT> d;
       d.occ = reinterpret_cast<typename Shape<N>::RowT*>(src);
       d.halo = reinterpret_cast<typename Shape<N>::RowT*>(src + S::P::kOcc);
@@ -452,17 +508,33 @@ k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
       d.vlist = reinterpret_cast<uint16_t*>(src + S::kVlOff);
       d.misc = reinterpret_cast<int*>(src + S::kMiscOff);
       d.lists = s_lists;
-      emit_runs<N, LAYOUT>(d, 0, emit_elems(d), (int)part, (int)parts, g0,
-                           [&](const uint32_t* list, int nf, uint32_t first) {
-        for (int r = 0, cnt = 0; r < nf; r += cnt) {
-          const unsigned long long g = g0 + first + (unsigned)r;
-          cnt = batch_faces<LAYOUT>(g, nf - r);
-          const int nw = faces_in(g, cnt, a.cap);
-          if (nw == 0) continue;
-          send(lane < nw ? list[r + lane] : 0u, nw, first + (uint32_t)r, g);
+      const int elems = emit_elems(d);
+      const unsigned runs = (unsigned)(elems + 32 * run_groups<N>() - 1) / (32u * run_groups<N>());
+      for (;;) {
+        unsigned run = 0;
+        if (lane == 0) {
+          run = atomicAdd(a.counts + i, 1u);
+          if (run == runs - 1u) {
+            atomicOr(a.counts + i, kTaken);
+            atomicSub(&a.ctl->open, 1u);
+          }
         }
-        __syncwarp();
-      });
+        run = __shfl_sync(0xffffffffu, run, 0);
+        if (run >= runs) break;
+        const int lo = (int)run * 32 * run_groups<N>();
+        emit_runs<N, LAYOUT>(d, lo, min(elems, lo + 32 * run_groups<N>()), 0, 1, g0,
+                             [&](const uint32_t* list, int nf, uint32_t first) {
+          for (int r = 0, cnt = 0; r < nf; r += cnt) {
+            const unsigned long long g = g0 + first + (unsigned)r;
+            cnt = batch_faces<LAYOUT>(g, nf - r);
+            const int nw = faces_in(g, cnt, a.cap);
+            if (nw == 0) continue;
+            const uint32_t q = lane < nw ? list[r + lane] : 0u;
+            store.template batch<false, true>(q, nw, first + (uint32_t)r, org, g, a.out0, a.out1);
+          }
+          __syncwarp();
+        });
+      }
     }
   }
   // The last CTA to finish resets the scan tickets and advances the epoch: every chunk of the

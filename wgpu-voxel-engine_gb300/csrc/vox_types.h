@@ -55,8 +55,10 @@ struct BatchCtl {
   unsigned int bar_count;  // grid barrier: CTAs arrived (reset by the last arriver)
   unsigned int bar_gen;    // grid barrier: generation, advanced by the last arriver
   unsigned int scan_flag;  // phased kernel: the generation whose offset scan is complete
-  unsigned int done;       // CTAs finished in a launch that mirrors its status (reset by the last)
+  unsigned int done;       // CTAs finished in a launch that mirrors its status, and in every
+                           // k_emit_lists (reset by the last)
   unsigned int next_scan;  // k_emit_lists: scan tickets (reset by its last CTA)
+  unsigned int open;       // list launches: chunks without a list whose runs are not all taken
 };
 
 // Gradients of the hashed 2-D lattice corners: entry A is the gradient (gx, gy) of p[p[A]].
@@ -88,7 +90,7 @@ struct MeshArgs {
   int spin_limit;                    // polls before a look-back wait gives up
   uint32_t* scratch;                 // phased/overlap kernels: per-chunk spilled chunk state
   int split;                         // phased/overlap kernels: emission segments per chunk
-  uint32_t* counts;                  // phased kernel: per-chunk face totals
+  uint32_t* counts;                  // per chunk: face total (phased), runs taken (list launches)
   int lane_flush;                    // staged faces leave shared memory by plain stores
   int lag;                           // overlap kernel: generation items ahead of emission
   unsigned* err_mirror;              // page-locked host word for the launch's status, or null

@@ -78,7 +78,7 @@ class BatchRun:
         sms = torch.cuda.get_device_properties(0).multi_processor_count
         return cfg.gen.kind != GEN_BERNOULLI and (
             cfg.chunk_size > 16 or cfg.gen.kind != GEN_HEIGHTMAP or cfg.layout != LAYOUT_VERTEX
-            or slab <= 2 * sms * (8 if cfg.chunk_size == 16 else 32))
+            or slab <= sms * (24 if cfg.chunk_size == 16 else 40))
 
     def launch(self):
         """One pass over the batch (asynchronous on the context's stream)."""
