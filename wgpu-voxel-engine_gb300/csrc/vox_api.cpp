@@ -127,7 +127,8 @@ struct vox_graph {
   uint32_t* d_counts = nullptr;           // phased: face totals (n)
   size_t state_bytes = 0;
   EpochWipe wipe;                         // by the context's launch count
-  int launches = 1;                       // kernel launches per replay (slabs of the batch)
+  int launches = 1;                       // batch launches per replay (slabs of the batch)
+  int kernels = 1;                        // kernels of one of them (lists: two)
   HaloScratch halo;                       // staged-halo buffers of the captured batch
 };
 
@@ -1439,6 +1440,7 @@ int vox_graph_capture(vox_ctx* ctx, const vox_chunk_coord* d_coords, const uint8
     g->wipe.wiped_at = ctx->launches;
     a.state = g->d_state;
   }
+  g->kernels = lists ? 2 : 1;
   // the graph owns its staged-halo buffers too (allocated before the capture)
   if (ctx->halo_staging && (st = ensure_halo(ctx, g->halo, (size_t)n)) != VOX_OK) return bail(st);
   // Capture on a private stream (thread-local mode: other threads' CUDA calls are not
@@ -1479,6 +1481,18 @@ int vox_graph_launch(vox_graph* g) {
     VOX_CUDA(ctx, cudaMemsetAsync(g->d_state, 0, g->state_bytes, ctx->stream), "cudaMemsetAsync(state)");
   VOX_CUDA(ctx, cudaGraphLaunch(g->exec, ctx->stream), "cudaGraphLaunch");
   return VOX_OK;
+}
+
+// Kernels of one batch launch: of a captured graph, or (g null) of the next vox_gen_mesh_batch of n
+// chunks with the context's tuning. For the Python package's launch counts; not in the public header.
+int voxgpu_batch_kernels(vox_ctx* ctx, int32_t n, const vox_graph* g) {
+  if (g) return g->kernels;
+  if (!ctx || n <= 0) return 0;
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  const int slab = slab_of(ctx, n);
+  const bool lists = use_lists(ctx, ctx->halo_staging ? GM_OCC : ctx->gm, slab, false) &&
+                     (size_t)slab * slot_bytes(ctx, true) < ctx->scratch.no_room;
+  return lists ? 2 : 1;
 }
 
 int vox_graph_destroy(vox_graph* g) {

@@ -9,8 +9,9 @@ memory comes from torch (plumbing only); every launch goes through the C ABI.
 """
 from __future__ import annotations
 
-from . import (GEN_BERNOULLI, GEN_HEIGHTMAP, LAYOUT_VERTEX, SCHEDULE_OVERLAP, VOX_OK,
-               VOX_ERR_CAPACITY, VoxError)
+import ctypes
+
+from . import VOX_OK, VOX_ERR_CAPACITY, VoxError
 
 
 class BatchRun:
@@ -59,26 +60,14 @@ class BatchRun:
             # staged halos: coordinate map (with the identity slots), neighbour lookup,
             # generation of the batch and (with neighbour masks) of the halo planes outside it
             self.launches_per_step += 3 + (1 if masks is not None else 0)
-        self.kernels_per_step = self.launches_per_step + (
-            (n + slab - 1) // slab if self._two_kernels(t, slab) else 0)
         self.graph = (ctx.capture_graph(self.d_coords, self.d_mask, n, self.out0, self.out1,
                                         self.cap, self.offsets, chunk_index_base=index_base)
                       if graph else None)
-
-    def _two_kernels(self, t, slab) -> bool:
-        """Whether a batch launch of `slab` chunks is two kernels (face lists, then records): the
-        library's rule (use_lists in csrc/vox_api.cpp), for counting."""
-        import torch
-        cfg = self.ctx.cfg
-        default = t.threads == {8: 64, 16: 256}.get(cfg.chunk_size, 512) and t.stage_faces == 32
-        if t.schedule != SCHEDULE_OVERLAP or not default or t.ctas_per_sm != 0:
-            return False
-        if t.halo_staging:
-            return True
-        sms = torch.cuda.get_device_properties(0).multi_processor_count
-        return cfg.gen.kind != GEN_BERNOULLI and (
-            cfg.chunk_size > 16 or cfg.gen.kind != GEN_HEIGHTMAP or cfg.layout != LAYOUT_VERTEX
-            or slab <= sms * (24 if cfg.chunk_size == 16 else 40))
+        # kernels: a batch launch is one or two (face lists, then records), as the library says
+        per_launch = ctx._lib.voxgpu_batch_kernels
+        per_launch.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p]
+        self.kernels_per_step = self.launches_per_step + (n + slab - 1) // slab * (
+            per_launch(ctx._h, n, self.graph._h if graph else None) - 1)
 
     def launch(self):
         """One pass over the batch (asynchronous on the context's stream)."""
