@@ -27,10 +27,13 @@ def test_kernels_per_step(vox, graph, n, kind, layout, count, tuning):
     run = BatchRun(ctx, coords, None if kind == "GEN_BERNOULLI" else [15] * count, graph=graph)
     run.launch()
     ctx.sync()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        run.launch()
-        ctx.sync()
-    kernels = [e for e in prof.events() if "k_" in e.name and "vox::" in e.name]
+    for _ in range(2):  # a process's first profile may come back empty
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            run.launch()
+            ctx.sync()
+        kernels = [e for e in prof.events() if "k_" in e.name and "vox::" in e.name]
+        if kernels:
+            break
     if not kernels:
         pytest.skip("no kernel activity from the profiler")
     assert run.kernels_per_step == len(kernels), [e.name for e in kernels]
