@@ -1220,6 +1220,7 @@ int vox_raster(vox_ctx* ctx, const float view_proj_colmajor[16], const void* d_v
       !d_depth_keys || !d_rgba || faces >= (1ull << 31) || (faces > 0 && (!d_vertices || !d_indices)))
     return fail(ctx, VOX_ERR_INVALID, "bad arguments");
   RasterArgs a;
+  a.num_sms = ctx->num_sms;
   a.vertices = d_vertices;
   a.indices = d_indices;
   a.faces = faces;

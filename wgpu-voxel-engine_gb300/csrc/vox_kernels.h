@@ -52,6 +52,7 @@ struct RasterArgs {
   int width, height;
   float m[16];              // global matrix, column-major
   uint32_t tex[6];          // texture index per face slot
+  int num_sms;              // of the device: the grid of the listed tiles
 };
 // Renders the faces into rgba (width x height x 4 bytes); keys: width x height u64.
 cudaError_t launch_raster(const RasterArgs& a, unsigned long long* keys, uint8_t* rgba,

@@ -360,7 +360,7 @@ cudaError_t launch_raster(const RasterArgs& a, unsigned long long* keys, uint8_t
     e = launch_dependent((const void*)k_raster_faces, dim3((unsigned)((a.faces + 127) / 128)), dim3(128),
                          with_list, 0, st);
     if (e == cudaSuccess && tiled)
-      e = launch_dependent((const void*)k_raster_tiles, dim3(152 * 8), dim3(256), with_list, 0, st);
+      e = launch_dependent((const void*)k_raster_tiles, dim3(a.num_sms * 8), dim3(256), with_list, 0, st);
   }
   if (e != cudaSuccess) return e;
   return launch_dependent((const void*)k_raster_shade, dim3((unsigned)((px + 255) / 256)), dim3(256),
