@@ -17,6 +17,8 @@ NVCC = os.path.join(_build._cuda_home(), "bin", "nvcc")
 
 pytestmark = pytest.mark.skipif(not os.path.exists(NVCC), reason="nvcc not found")
 
+SPILL_LOADS = {}  # kernel (mangled): spill load bytes
+
 
 def compile_units(units, tmp_path):
     """{unit: {kernel (mangled): [registers, spill store bytes]}}, the units compiled in
@@ -41,6 +43,9 @@ def compile_units(units, tmp_path):
             m = re.search(r"(\d+) bytes spill stores", line)
             if m and name:
                 res[name][1] = int(m.group(1))
+            m = re.search(r"(\d+) bytes spill loads", line)
+            if m and name:
+                SPILL_LOADS[name] = int(m.group(1))
             m = re.search(r"Used (\d+) registers", line)
             if m and name:
                 res[name][0] = int(m.group(1))
@@ -106,3 +111,38 @@ def test_heightmap_generation_budget(n16):
 @pytest.mark.parametrize("layout", [0, 1])
 def test_stress_64_kernels_fit_two_ctas_of_512(n64, stem, layout):
     assert find(n64, stem, 64, 3, layout, 512)[0] <= 64
+
+
+def resources(res, stem, *params):
+    """Registers, spill store and spill load bytes of stem<params...>."""
+    entry = find(res, stem, *params)
+    name = next(k for k in res if res[k] is entry)
+    return entry[0], entry[1], SPILL_LOADS[name]
+
+
+@pytest.mark.parametrize("gm", [0, 1, 2])  # resident occupancy; heightmap; density
+@pytest.mark.parametrize("n,big", [(16, 0), (32, 0), (32, 1), (64, 0), (64, 1)])
+def test_list_chunks_keep_their_budget(units, n, gm, big):
+    """32 registers a thread up to 32^3 without density noise, else 64 (see list_min_ctas), and no
+    spills but a few bytes around the per-sample fallback of the noise."""
+    regs, stores, loads = resources(units[f"vox_kernels_n{n}.cu"], "k_list_chunks", n, gm, big)
+    assert regs <= (64 if gm == 2 or n == 64 else 32)
+    if gm == 2 or (gm == 1 and n == 64):
+        assert stores <= 24 and loads <= 64
+    else:
+        assert stores == 0 and loads == 0
+
+
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("n", [16, 32, 64])
+def test_emission_keeps_32_warps_per_sm(units, n, layout):
+    regs, stores, loads = resources(units[f"vox_kernels_n{n}.cu"], "k_emit_lists", n, layout)
+    assert regs <= 64
+    assert (stores, loads) == (0, 0) if layout == 1 else (stores <= 40 and loads <= 96)
+
+
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("n", [16, 32, 64])
+def test_single_chunk_mesher_does_not_spill(units, n, layout):
+    regs, stores, loads = resources(units[f"vox_kernels_n{n}.cu"], "k_mesh_single", n, layout)
+    assert regs <= 64 and stores == 0 and loads == 0
