@@ -453,7 +453,8 @@ k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
   while (ok) {
     int i = (int)(k >> a.split);
     const unsigned part = k & (parts - 1u);
-    if (k < items) {
+    const bool own = k < items;
+    if (own) {
       k += stride;
     } else {
       if (met < 0) break;
@@ -474,7 +475,8 @@ k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
       else store.template batch<false>(q, nw, first, org, g, a.out0, a.out1);
     };
     unsigned char* src = reinterpret_cast<unsigned char*>(a.scratch) + (unsigned long long)i * S::kBytes;
-    if (total <= S::kCap) {  // (never of an open chunk)
+    if (total <= S::kCap) {
+      if (!own) continue;  // (its count was not there yet; it is now, and not open)
       // the output lines that the chunk touches, cut evenly over the parts
       const uint32_t* codes = reinterpret_cast<const uint32_t*>(src);
       const unsigned phase = (unsigned)(g0 & (unsigned long long)(kLine - 1u));
@@ -510,6 +512,7 @@ k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
       d.lists = s_lists;
       const int elems = emit_elems(d);
       const unsigned runs = (unsigned)(elems + 32 * run_groups<N>() - 1) / (32u * run_groups<N>());
+      bool took = false;
       for (;;) {
         unsigned run = 0;
         if (lane == 0) {
@@ -520,7 +523,11 @@ k_emit_lists(const __grid_constant__ MeshArgs a, const __grid_constant__ TablesD
           }
         }
         run = __shfl_sync(0xffffffffu, run, 0);
-        if (run >= runs) break;
+        if (run >= runs) {
+          if (!own && !took) done += 32u;  // all taken meanwhile: go on behind it
+          break;
+        }
+        took = true;
         const int lo = (int)run * 32 * run_groups<N>();
         emit_runs<N, LAYOUT>(d, lo, min(elems, lo + 32 * run_groups<N>()), 0, 1, g0,
                              [&](const uint32_t* list, int nf, uint32_t first) {
