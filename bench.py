@@ -57,10 +57,10 @@ L2_FLUSH_BYTES = 256 << 20
 # to the launch's chunk count (DRAM bytes grow with the faces written).
 NCU = {
     ("k_list_chunks + k_emit_lists", "heightmap"): {
-        "traffic": 9170000, "warp_instructions": 13748599, "chunks": 1024, "per_step": True,
+        "traffic": 8600000, "warp_instructions": 13640000, "chunks": 1024, "per_step": True,
         "summary": "profiles/face_lists.md"},
     ("k_list_chunks + k_emit_lists", "density"): {
-        "traffic": 617600000, "warp_instructions": 143786463, "chunks": 4096, "per_step": True,
+        "traffic": 615400000, "warp_instructions": 152150000, "chunks": 4096, "per_step": True,
         "summary": "profiles/face_lists.md"},
     ("k_mesh_batch_overlap", "heightmap"): {
         "traffic": 7112704, "warp_instructions": 18389229, "chunks": 1024,

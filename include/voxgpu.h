@@ -237,10 +237,10 @@ int vox_gen_mesh_host(vox_ctx* ctx, const vox_chunk_coord* h_coords, const uint8
 
 /* ---- Tuning ------------------------------------------------------------------------------ */
 
-/* Launch shape of the meshing kernels. With the shape of an untuned context (vox_ctx_get_tuning
- * after vox_ctx_create) the overlap schedule into device memory is two launches (face lists, then
- * records) with shapes of their own, where these are the faster way; every other shape is that of
- * one persistent launch. */
+/* Launch shape of the batch meshing kernels (vox_mesh has one of its own, for every tuning). With
+ * the shape of an untuned context (vox_ctx_get_tuning after vox_ctx_create) the overlap schedule
+ * into device memory is two launches (face lists, then records) with shapes of their own, where
+ * these are the faster way; every other shape is that of one persistent launch. */
 typedef struct vox_tuning {
   int32_t threads;     /* CTA size; each chunk size has two (8: 32/64, 16: 128/256,
                           32: 256/512, 64: 512/1024) */

@@ -425,8 +425,8 @@ int check_outputs(vox_ctx* ctx, void* out0, void* out1, uint64_t cap) {
 // in 2^a.split parts, a warp each: enough to give every resident warp one part (two from 32^3 on,
 // whose chunks are less even), but no fewer than one per 8 (up to 16^3) or 16 output lines
 // of a chunk with two faces a column, and no more than one per 2 or 4 lines. Measured, us a batch
-// with 2, 4, 8, 16, 32 parts: 1024 terrain chunks of 16^3 41, 35, 34, 34, 38; 777 cave chunks
-// of 32^3 from occupancy 56, 51, 46, 42, 41; 64 chunks of 32^3, instances 34, 27, 23, 22, 21.
+// with 2, 4, 8, 16, 32 parts: 1024 terrain chunks of 16^3 41, 32, 31, 31, 35; 777 cave chunks
+// of 32^3 from occupancy 50, 47, 40, 37, 38; 64 chunks of 32^3, instances 25, 19, 16, 15, 15.
 int issue_lists(vox_ctx* ctx, MeshArgs& a, int gm, cudaStream_t stream) {
   const KernelSet& ks = *ctx->ks;
   const int warps = ks.emit_threads / 32, N = ks.n_size;

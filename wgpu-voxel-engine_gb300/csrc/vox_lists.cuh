@@ -11,11 +11,12 @@
 // launch is a programmatic dependent of the first (its CTAs start as soon as the last
 // generation CTA has started, and wait for chunks, not for the kernel), so splitting costs no
 // launch gap.
-// Measured, us a batch, one launch -> two: 1024 terrain chunks of 16^3 39.6 -> 33.9, 64 start
-// chunks of 32^3 as instances 41.6 -> 21.7, 777 cave chunks of 32^3 from occupancy 62 -> 42,
-// 4096 cave chunks generated 285 -> 279. What bounds them: generation by its instructions
-// (57 % of issue at 16^3), emission by the offsets' way (the slowest chunk of a group, its scan,
-// the poll: about 4 us) and then the writes (61 MB in 11 us into L2, 4.4 TB/s into HBM).
+// Measured, us a batch, one launch -> two (both as they are now): 1024 terrain chunks of 16^3 33.7 ->
+// 30.7, 64 start chunks of 32^3 as instances 37.2 -> 16.1, 777 cave chunks of 32^3 from occupancy
+// 53.8 -> 35.4, 4096 cave chunks generated 301 -> 282. What bounds them: generation by its
+// instructions (58 % of issue at 16^3), emission by the offsets' way (the slowest chunk of a group, its
+// scan, the poll: about 4 us) and then the writes (61 MB in 11 us into L2, 4.7 TB/s into HBM).
+// Figures beside single choices below were taken when the choice was made, each pair on one tree.
 #pragma once
 
 #include "vox_device.cuh"
